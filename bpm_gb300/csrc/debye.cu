@@ -115,6 +115,24 @@ __device__ __forceinline__ float coord_f32(int i, float x1, float x2, int N) {
 
 constexpr double kTwoPi = 6.283185307179586, kInvTwoPi = 0.15915494309189535;
 
+// An FP64 value v as a float pair (hi, lo): hi = v rounded to FP32, lo = v - hi rounded to FP32,
+// so hi + lo is v to about 2^-48 relative.
+__host__ __device__ __forceinline__ float2 split_pair(double v) {
+  const float hi = (float)v;
+  return make_float2(hi, (float)(v - (double)hi));
+}
+
+// a * b of two float pairs, rounded once to FP32: the exact rounding error of a.hi b.hi (an
+// FMA) plus the cross terms, added to the rounded product (a.lo b.lo is below 2^-48). The
+// result is the FP32 rounding of the FP64 product except where that product lies within
+// about 2^-46 of a rounding boundary; it takes FP32 instructions instead of two of the FP64
+// pipe, which runs at 1/64 of the FP32 rate on this GPU.
+__device__ __forceinline__ float mul_pair(float2 a, float2 b) {
+  const float p = __fmul_rn(a.x, b.x);
+  const float e = fmaf(a.x, b.x, -p);
+  return __fadd_rn(p, fmaf(a.x, b.y, fmaf(a.y, b.x, e)));
+}
+
 // trapezoid node idx of its annulus (psf_debye.cl:62-78), FP64: sin t, cos t and the pupil
 // weight w
 __device__ __forceinline__ void node_values(const NodeArgs& a, int idx, double& s, double& c, double& w) {
@@ -213,24 +231,56 @@ __host__ __device__ constexpr double hankel_a(int n, int k) {
   return a;
 }
 
-// J2 from J0, J1: ascending series for small x, the three-term recurrence J2 = 2 J1/x - J0
-// otherwise (stable for n = 2 < x).
-__device__ __forceinline__ float bessel_j2(float x, float j0, float j1) {
-  const float ax = fabsf(x);
-  if (ax < 4.f) {
-    // J2(x) = sum_k (-1)^k (x/2)^(2k+2) / (k! (k+2)!)
-    const float q = 0.25f * x * x;
-    float term = 0.5f * q;  // k = 0: (x/2)^2 / 2!
-    float sum = term;
-#pragma unroll
-    for (int k = 1; k < 12; k++) {
-      term *= -q * (1.f / (float)(k * (k + 2)));  // the reciprocal folds to a constant
-      sum += term;
-    }
-    return sum;
+// Taylor coefficients of J0 and J2 for 0 <= x < 16 in intervals of width 1/4: row i covers
+// [i/4, i/4 + 1/4) about its middle (row 0 about x = 0, so that J1 and J2 keep their relative
+// accuracy there), c[0..1][i] the eight coefficients of J0, c[2..3][i] those of J2, lowest
+// power first. Values at the middle come from the power series in FP64, the higher
+// coefficients from Bessel's equation x^2 y'' + x y' + (x^2 - n^2) y = 0 written about it.
+constexpr int BT_ROWS = 64;
+constexpr float BT_END = 16.f;
+struct BesselTaylor {
+  float4 c[4][BT_ROWS];
+};
+
+constexpr double bessel_series(int n, double x) {  // sum_k (-1)^k (x/2)^(2k+n) / (k! (k+n)!)
+  double term = 1.;
+  for (int j = 1; j <= n; j++) term *= .5 * x / j;
+  double sum = term;
+  for (int k = 1; k < 60; k++) {
+    term *= -.25 * x * x / ((double)k * (k + n));
+    sum += term;
   }
-  return 2.f * j1 / x - j0;
+  return sum;
 }
+
+constexpr BesselTaylor bessel_taylor() {
+  BesselTaylor t{};
+  for (int i = 0; i < BT_ROWS; i++) {
+    double a[8] = {}, b[8] = {};
+    if (i == 0) {
+      a[0] = 1., a[2] = -1. / 4., a[4] = 1. / 64., a[6] = -1. / 2304.;
+      b[2] = 1. / 8., b[4] = -1. / 96., b[6] = 1. / 3072.;
+    } else {
+      const double c = .25 * i + .125;
+      const double j1 = bessel_series(1, c);
+      a[0] = bessel_series(0, c), a[1] = -j1;
+      b[0] = bessel_series(2, c), b[1] = j1 - 2. * b[0] / c;
+      for (int n = 0; n < 4; n += 2) {
+        double* y = n ? b : a;
+        for (int m = 0; m < 6; m++)
+          y[m + 2] = -(c * (m + 1.) * (2. * m + 1.) * y[m + 1] + (m * m + c * c - n * n) * y[m] +
+                       (m > 0 ? 2. * c * y[m - 1] : 0.) + (m > 1 ? y[m - 2] : 0.)) /
+                     (c * c * (m + 2.) * (m + 1.));
+      }
+    }
+    t.c[0][i] = float4{(float)a[0], (float)a[1], (float)a[2], (float)a[3]};
+    t.c[1][i] = float4{(float)a[4], (float)a[5], (float)a[6], (float)a[7]};
+    t.c[2][i] = float4{(float)b[0], (float)b[1], (float)b[2], (float)b[3]};
+    t.c[3][i] = float4{(float)b[4], (float)b[5], (float)b[6], (float)b[7]};
+  }
+  return t;
+}
+__device__ const BesselTaylor g_bessel = bessel_taylor();
 
 // J0, J1 and J2 together. From x = 16 on, the expansion above truncated after x^-7 (its
 // error, below 2e-9 of the envelope sqrt(2 / (pi x)), is under FP32 rounding), with one
@@ -238,14 +288,27 @@ __device__ __forceinline__ float bessel_j2(float x, float j0, float j1) {
 // (cos x + sin x) / sqrt 2, sin chi_0 = (sin x - cos x) / sqrt 2, cos chi_1 = sin chi_0,
 // sin chi_1 = -cos chi_0; 1/x and the envelope come from the approximate reciprocal and
 // reciprocal square root (2 ulp, far below what the truncated series resolves), and J2 from
-// the recurrence 2 J1/x - J0 with that reciprocal. Below 16: CUDA's j0f and j1f, J2 by
-// bessel_j2.
+// the recurrence 2 J1/x - J0 with that reciprocal. Below 16 the Taylor polynomials of
+// g_bessel, J1 as minus the derivative of J0's: no branch and no division, absolute errors
+// below 1e-7 against FP64 over [0, 16).
 __device__ __forceinline__ void bessel_j012(float x, float& j0, float& j1, float& j2) {
   const float ax = fabsf(x);
-  if (ax < 16.f) {
-    j0 = j0f(x);
-    j1 = j1f(x);
-    j2 = bessel_j2(x, j0, j1);
+  if (ax < BT_END) {
+    const int i = (int)(ax * 4.f);
+    const float4 a = __ldg(&g_bessel.c[0][i]), b = __ldg(&g_bessel.c[1][i]);
+    const float4 e = __ldg(&g_bessel.c[2][i]), f = __ldg(&g_bessel.c[3][i]);
+    const float d = ax - (i > 0 ? fmaf(.25f, (float)i, .125f) : 0.f);
+    // value p and derivative q of J0's polynomial in one pass
+    float p = b.w, q = b.w;
+    p = fmaf(p, d, b.z), q = fmaf(q, d, p);
+    p = fmaf(p, d, b.y), q = fmaf(q, d, p);
+    p = fmaf(p, d, b.x), q = fmaf(q, d, p);
+    p = fmaf(p, d, a.w), q = fmaf(q, d, p);
+    p = fmaf(p, d, a.z), q = fmaf(q, d, p);
+    p = fmaf(p, d, a.y), q = fmaf(q, d, p);
+    j0 = fmaf(p, d, a.x);
+    j1 = x < 0.f ? q : -q;
+    j2 = fmaf(fmaf(fmaf(fmaf(fmaf(fmaf(fmaf(f.w, d, f.z), d, f.y), d, f.x), d, e.w), d, e.z), d, e.y), d, e.x);
     return;
   }
   const float r = __fdividef(1.f, ax), y = r * r;
@@ -616,32 +679,94 @@ int launch_assemble(const debye_desc* d, bool gauss, const OctGeom& g, int M, in
 
 // Fields at arbitrary points (debye_wolf_at, psf_debye.cl:187-269) or on one z plane
 // (debye_wolf_plane, :117-183). Without a grid in z the quadrature does not factorise into
-// a matrix product, so each thread sums its point's integrand over the nodes, as the
-// reference does, with the node tables staged through shared memory. On the plane the
-// phase e^{i kz cos t} is one table over the nodes; at free points the argument kz cos t
-// is formed and reduced modulo 2 pi in FP64 and the reduced angle goes through sincosf.
+// a matrix product, so every point sums its integrand over the nodes, as the reference does.
+// On the plane the phase e^{i kz cos t} is one table over the nodes; at free points the
+// argument kz cos t is formed as a float pair and reduced modulo 2 pi before sincosf.
 struct PointArgs {
   long long n;
   int nx, ny;  // plane grid (GRID only)
   float x1, x2, y1, y2;
   double k;
+  float2 k2;   // k as a float pair
   float ex0, ey0;
   int T;
 };
 
 constexpr int PT_THREADS = 128, PT_CHUNK = 256;
 
+// Node tables of the point kernel, one node per thread in 32-thread blocks (FP64 chains on as
+// many SMs as possible): nd = (sin t, p_0, p_1, p_2) and aux = e^{i kz cos t} on a plane
+// (PLANE), cos t as a float pair (and in FP64 in ct) otherwise.
+template <bool PLANE>
+__global__ void debye_point_nodes_kernel(NodeArgs a, double kz, float4* nd, float2* aux, double* ct, int T) {
+  dep_release();
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= T) return;
+  double s, c, w;
+  node_values(a, idx, s, c, w);
+  nd[idx] = make_float4((float)s, (float)(w * (c + 1.)), (float)(w * s), (float)(w * (c - 1.)));
+  if (PLANE) {
+    double sn, cs;
+    sincos(kz * c, &sn, &cs);
+    aux[idx] = make_float2((float)cs, (float)sn);
+  } else {
+    aux[idx] = split_pair(c);
+    ct[idx] = c;
+  }
+}
+
+// k r rounded to FP32: r^2 and r as float pairs (the error of each square by an FMA, one
+// Newton correction of the root), in FP64 where the squares would leave the FP32 range
+__device__ __forceinline__ float point_kr(float x, float y, const PointArgs& a) {
+  if (x == 0.f && y == 0.f) return 0.f;
+  const float m = fmaxf(fabsf(x), fabsf(y));
+  if (!(m > 1e-12f && m < 1e15f)) {
+    const double xd = x, yd = y;
+    return (float)(a.k * sqrt(xd * xd + yd * yd));
+  }
+  const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), s = __fadd_rn(xx, yy);
+  const float bb = __fsub_rn(s, xx);
+  const float lo = (__fsub_rn(xx, __fsub_rn(s, bb)) + __fsub_rn(yy, bb)) + (fmaf(x, x, -xx) + fmaf(y, y, -yy));
+  const float h = __fsqrt_rn(s);
+  return mul_pair(make_float2(h, __fdividef(fmaf(-h, h, s) + lo, 2.f * h)), a.k2);
+}
+
+// e^{i kz c} of a float pair c: the product as a pair (p, e), p reduced modulo 2 pi with the
+// two leading parts of 2 pi (q 2 pi_hi and the difference are exact in the FMA for |p| <=
+// 2^20), in FP64 (kzd * *cd) beyond
+__device__ __forceinline__ float2 point_phase(float2 kz, float2 c, double kzd, const double* cd) {
+  const float p = __fmul_rn(kz.x, c.x);
+  float ang;
+  if (fabsf(p) <= 1048576.f) {
+    const float e = fmaf(kz.x, c.x, -p) + fmaf(kz.x, c.y, kz.y * c.x);
+    const float q = rintf(p * (float)kInvTwoPi);
+    constexpr float hi = (float)kTwoPi, lo = (float)(kTwoPi - (double)(float)kTwoPi);
+    ang = fmaf(-q, hi, p) + fmaf(-q, lo, e);
+  } else {
+    const double arg = kzd * *cd;
+    ang = (float)fma(-rint(arg * kInvTwoPi), kTwoPi, arg);
+  }
+  float2 r;
+  sincosf(ang, &r.y, &r.x);
+  return r;
+}
+
+// 2^lg neighbouring lanes share a point: lane j takes the nodes j, j + 2^lg, ... and the six
+// sums are added by shuffles. The kernel is bound by the chain of Bessel evaluations per
+// thread and by how many threads there are: with one thread per point a 128 x 128 plane is
+// 4 warps on each SM and 4000 points are 32 blocks on 152 SMs. GB300, 201 nodes, whole
+// call: 128 x 128 plane 105 -> 37 us, 4000 free points 166 -> 67 us (one thread per point,
+// j0f/j1f and FP64 phase and azimuth before).
 template <bool GRID>
 __global__ void __launch_bounds__(PT_THREADS) debye_points_kernel(
-    PointArgs a, const float* __restrict__ xs, const float* __restrict__ ys, const float* __restrict__ zs,
-    const double* __restrict__ si, const double* __restrict__ ct, const float* __restrict__ wf,
-    const float2* __restrict__ Et, float* __restrict__ u, float2* __restrict__ ex, float2* __restrict__ ey,
-    float2* __restrict__ ez) {
-  __shared__ float s_si[PT_CHUNK];
-  __shared__ float s_w[3][PT_CHUNK];
-  __shared__ double s_ct[GRID ? 1 : PT_CHUNK];
-  __shared__ float2 s_E[GRID ? PT_CHUNK : 1];
-  const long long p = (long long)blockIdx.x * PT_THREADS + threadIdx.x;
+    PointArgs a, int lg, const float* __restrict__ xs, const float* __restrict__ ys, const float* __restrict__ zs,
+    const float4* __restrict__ nd, const float2* __restrict__ aux, const double* __restrict__ ct,
+    float* __restrict__ u, float2* __restrict__ ex, float2* __restrict__ ey, float2* __restrict__ ez) {
+  __shared__ float4 s_nd[PT_CHUNK];
+  __shared__ float2 s_aux[PT_CHUNK];
+  const long long gid = (long long)blockIdx.x * PT_THREADS + threadIdx.x;
+  const long long p = gid >> lg;
+  const int step = 1 << lg, sub = (int)gid & (step - 1);
   const bool active = p < a.n;
   float x = 0.f, y = 0.f, z = 0.f;
   if (active) {
@@ -655,39 +780,27 @@ __global__ void __launch_bounds__(PT_THREADS) debye_points_kernel(
       z = zs[p];
     }
   }
-  const double xd = x, yd = y;
-  const float kr = (float)(a.k * sqrt(xd * xd + yd * yd));
-  const double kz = a.k * (double)z;
+  const float kr = point_kr(x, y, a);
+  const double kzd = GRID ? 0. : a.k * (double)z;
+  const float2 kz = GRID ? make_float2(0.f, 0.f) : split_pair(kzd);
   float2 I0 = make_float2(0.f, 0.f), I1 = I0, I2 = I0;
+  dep_wait();  // the node tables; the points were there before that launch
   for (int t0 = 0; t0 < a.T; t0 += PT_CHUNK) {
     const int nt = min(PT_CHUNK, a.T - t0);
     __syncthreads();
     for (int e = threadIdx.x; e < nt; e += PT_THREADS) {
-      s_si[e] = (float)si[t0 + e];
-      s_w[0][e] = wf[t0 + e];
-      s_w[1][e] = wf[a.T + t0 + e];
-      s_w[2][e] = wf[2 * a.T + t0 + e];
-      if (GRID)
-        s_E[e] = Et[t0 + e];
-      else
-        s_ct[e] = ct[t0 + e];
+      s_nd[e] = nd[t0 + e];
+      s_aux[e] = aux[t0 + e];
     }
     __syncthreads();
     if (!active) continue;
-    for (int tt = 0; tt < nt; tt++) {
-      const float xb = kr * s_si[tt];
-      float j0, j1;
-      float j2;
-      bessel_j012(xb, j0, j1, j2);
-      float2 e;
-      if (GRID) {
-        e = s_E[tt];
-      } else {
-        const double arg = kz * s_ct[tt];
-        const double q = rint(arg * kInvTwoPi);
-        sincosf((float)fma(-q, kTwoPi, arg), &e.y, &e.x);
-      }
-      const float a0 = s_w[0][tt] * j0, a1 = s_w[1][tt] * j1, a2 = s_w[2][tt] * j2;
+#pragma unroll 2
+    for (int tt = sub; tt < nt; tt += step) {
+      const float4 w = s_nd[tt];
+      float j0, j1, j2;
+      bessel_j012(kr * w.x, j0, j1, j2);
+      const float2 e = GRID ? s_aux[tt] : point_phase(kz, s_aux[tt], kzd, ct + t0 + tt);
+      const float a0 = w.y * j0, a1 = w.z * j1, a2 = w.w * j2;
       I0.x = fmaf(a0, e.x, I0.x);
       I0.y = fmaf(a0, e.y, I0.y);
       I1.x = fmaf(a1, e.x, I1.x);
@@ -696,12 +809,26 @@ __global__ void __launch_bounds__(PT_THREADS) debye_points_kernel(
       I2.y = fmaf(a2, e.y, I2.y);
     }
   }
-  if (!active) return;
-  const double phi = atan2(yd, xd);
-  double s1d, c1d, s2d, c2d;
-  sincos(phi, &s1d, &c1d);
-  sincos(2. * phi, &s2d, &c2d);
-  const float c1 = (float)c1d, s1 = (float)s1d, c2 = (float)c2d, s2 = (float)s2d;
+  for (int o = step >> 1; o > 0; o >>= 1) {
+    I0.x += __shfl_xor_sync(0xffffffffu, I0.x, o);
+    I0.y += __shfl_xor_sync(0xffffffffu, I0.y, o);
+    I1.x += __shfl_xor_sync(0xffffffffu, I1.x, o);
+    I1.y += __shfl_xor_sync(0xffffffffu, I1.y, o);
+    I2.x += __shfl_xor_sync(0xffffffffu, I2.x, o);
+    I2.y += __shfl_xor_sync(0xffffffffu, I2.y, o);
+  }
+  if (!active || sub != 0) return;
+  // azimuth from the coordinates scaled by their larger one (phi = 0 at the origin):
+  // cos phi = x/r, sin phi = y/r, cos 2 phi = (x-y)(x+y)/r^2, sin 2 phi = 2xy/r^2
+  float c1 = 1.f, s1 = 0.f, c2 = 1.f, s2 = 0.f;
+  const float m = fmaxf(fabsf(x), fabsf(y));
+  if (m > 0.f) {
+    const float xm = x / m, ym = y / m, r2 = fmaf(xm, xm, ym * ym), ir = rsqrtf(r2);
+    c1 = xm * ir;
+    s1 = ym * ir;
+    c2 = (xm - ym) * (xm + ym) / r2;
+    s2 = 2.f * xm * ym / r2;
+  }
   const float ex0 = a.ex0, ey0 = a.ey0;
   // psf_debye.cl:254-263
   const float2 vx = make_float2(ex0 * (I0.x + I2.x * c2) + (ey0 * s2) * I2.x,
@@ -712,7 +839,6 @@ __global__ void __launch_bounds__(PT_THREADS) debye_points_kernel(
   const float pz = ex0 * c1 + ey0 * s1;
   if (ez) ez[p] = make_float2(2.f * I1.y * pz, -2.f * I1.x * pz);
 }
-
 
 // ---------------------------------------------------------------------------------------
 // Tensor-core quadrature. Operands are K-major (node index t contiguous) so TMA tiles of
@@ -736,24 +862,6 @@ __device__ __forceinline__ int radius_column(int r, int nxo, bool sym) {
   while ((b + 1) * (b + 2) / 2 <= r) b++;
   const int a = r - b * (b + 1) / 2;
   return b * nxo + a;
-}
-
-// An FP64 value v as a float pair (hi, lo): hi = v rounded to FP32, lo = v - hi rounded to FP32,
-// so hi + lo is v to about 2^-48 relative.
-__device__ __forceinline__ float2 split_pair(double v) {
-  const float hi = (float)v;
-  return make_float2(hi, (float)(v - (double)hi));
-}
-
-// a * b of two float pairs, rounded once to FP32: the exact rounding error of a.hi b.hi (an
-// FMA) plus the cross terms, added to the rounded product (a.lo b.lo is below 2^-48). The
-// result is the FP32 rounding of the FP64 product except where that product lies within
-// about 2^-46 of a rounding boundary; it takes FP32 instructions instead of two of the FP64
-// pipe, which runs at 1/64 of the FP32 rate on this GPU.
-__device__ __forceinline__ float mul_pair(float2 a, float2 b) {
-  const float p = __fmul_rn(a.x, b.x);
-  const float e = fmaf(a.x, b.x, -p);
-  return __fadd_rn(p, fmaf(a.x, b.y, fmaf(a.y, b.x, e)));
 }
 
 // Nodes and radii of the tensor-core path in one launch: blocks [0, nbn) one quadrature node
@@ -1337,7 +1445,7 @@ int run_octant(const debye_desc* d, bool gauss, double sig, float* u, void* ex, 
 }
 
 struct PointsLayout {
-  size_t si, ct, wf, E, total;
+  size_t nd, aux, ct, total;
   int T;
 };
 
@@ -1345,12 +1453,19 @@ PointsLayout points_layout(const debye_desc* d) {
   PointsLayout L;
   L.T = (d->n_na / 2) * (d->n_integration_steps + 1);
   size_t off = 0;
-  L.si = off; off += align256(sizeof(double) * L.T);
+  L.nd = off; off += align256(sizeof(float4) * L.T);
+  L.aux = off; off += align256(sizeof(float2) * L.T);
   L.ct = off; off += align256(sizeof(double) * L.T);
-  L.wf = off; off += align256(sizeof(float) * 3 * L.T);
-  L.E = off; off += align256(sizeof(float2) * L.T);
-  L.total = off;
+  L.total = off + 256;  // room to align the tables to 16 bytes inside any workspace
   return L;
+}
+
+// lanes per point (as a power of two): enough that the points fill the device with 32 warps
+// on each of 152 SMs, at most a warp, and no more than there are nodes
+int point_lanes_log2(long long n, int T) {
+  int lg = 0;
+  while (lg < 5 && (n << lg) < 152LL * 1024 && (2 << lg) <= T) lg++;
+  return lg;
 }
 
 // shared by focus_field_debye_plane (GRID) and focus_field_debye_at
@@ -1361,25 +1476,24 @@ int run_points(const debye_desc* d, bool grid, double zplane, const float* xs, c
     set_error("workspace too small: need " + std::to_string(L.total) + " bytes");
     return BPM_ERR_OOM;
   }
-  char* w = static_cast<char*>(ws);
-  double* si = reinterpret_cast<double*>(w + L.si);
+  char* w = reinterpret_cast<char*>(((uintptr_t)ws + 15) & ~uintptr_t(15));
+  float4* nd = reinterpret_cast<float4*>(w + L.nd);
+  float2* aux = reinterpret_cast<float2*>(w + L.aux);
   double* ct = reinterpret_cast<double*>(w + L.ct);
-  float* wf = reinterpret_cast<float*>(w + L.wf);
-  float2* E = reinterpret_cast<float2*>(w + L.E);
   NodeArgs na = node_args(d, W_SINE);
-  const double k = wave_number(d);
-  debye_nodes_kernel<<<(L.T + 127) / 128, 128, 0, s>>>(na, si, ct, wf, L.T);
-  BPM_LAUNCH_CHECK("debye_nodes_kernel");
   PointArgs a;
   memset(&a, 0, sizeof(a));
   a.n = n;
-  a.k = k;
+  a.k = wave_number(d);
+  a.k2 = split_pair(a.k);
   a.ex0 = (float)d->ex0;
   a.ey0 = (float)d->ey0;
   a.T = L.T;
   if (n == 0) return BPM_OK;
-  const long long blocks = (n + PT_THREADS - 1) / PT_THREADS;
+  const int lg = point_lanes_log2(n, L.T);
+  const long long blocks = ((n << lg) + PT_THREADS - 1) / PT_THREADS;
   if (blocks > 0x7fffffffLL) { set_error("too many points"); return BPM_ERR_SHAPE; }
+  const unsigned nb = (unsigned)((L.T + 31) / 32);
   if (grid) {
     // _focus_fields_debye.py:201-209: x in [-(Nx//2) dx, (Nx - Nx//2) dx], float32
     a.nx = d->nx;
@@ -1388,18 +1502,15 @@ int run_points(const debye_desc* d, bool grid, double zplane, const float* xs, c
     a.x2 = (float)((double)(d->nx - d->nx / 2) * d->dx);
     a.y1 = (float)(-(double)(d->ny / 2) * d->dy);
     a.y2 = (float)((double)(d->ny - d->ny / 2) * d->dy);
-    debye_phase_kernel<<<(L.T + 127) / 128, 128, 0, s>>>(1, 1, (float)zplane, 0.f, k, ct, E, L.T);
-    BPM_LAUNCH_CHECK("debye_phase_kernel");
-    debye_points_kernel<true><<<(unsigned)blocks, PT_THREADS, 0, s>>>(a, nullptr, nullptr, nullptr, si, ct, wf, E,
-                                                                      u, static_cast<float2*>(ex),
-                                                                      static_cast<float2*>(ey),
-                                                                      static_cast<float2*>(ez));
+    debye_point_nodes_kernel<true><<<nb, 32, 0, s>>>(na, a.k * (double)(float)zplane, nd, aux, ct, L.T);
   } else {
-    debye_points_kernel<false><<<(unsigned)blocks, PT_THREADS, 0, s>>>(a, xs, ys, zs, si, ct, wf, E, u,
-                                                                       static_cast<float2*>(ex),
-                                                                       static_cast<float2*>(ey),
-                                                                       static_cast<float2*>(ez));
+    debye_point_nodes_kernel<false><<<nb, 32, 0, s>>>(na, 0., nd, aux, ct, L.T);
   }
+  BPM_LAUNCH_CHECK("debye_point_nodes_kernel");
+  BPM_CUDA_TRY(launch_dep(grid ? debye_points_kernel<true> : debye_points_kernel<false>, dim3((unsigned)blocks),
+                          dim3(PT_THREADS), 0, s, a, lg, xs, ys, zs, (const float4*)nd, (const float2*)aux,
+                          (const double*)ct, u, static_cast<float2*>(ex), static_cast<float2*>(ey),
+                          static_cast<float2*>(ez)));
   BPM_LAUNCH_CHECK("debye_points_kernel");
   return BPM_OK;
 }

@@ -158,6 +158,30 @@ def test_at_oracle_parity_and_grid_consistency(bpm):
     assert res_d[1].is_cuda and np.array_equal(res_d[1].cpu().numpy(), res[1])
 
 
+@pytest.mark.parametrize("n,steps", [(1, 2), (3, 40), (33, 31), (1000, 255), (9000, 256), (170000, 20)])
+def test_at_lanes_per_point(bpm, n, steps):
+    """Free points from one to more than a device full of threads (a point takes 32 lanes down
+    to one), node counts around the lanes and the staged chunk of 256, with points on the
+    axis and, for the larger sets, one so far away that its phase leaves the float-pair
+    reduction. Against the FP64 oracle, per point: with S the sum of the node magnitudes (ex
+    at the focus), every term is off by at most 6e-7 of its magnitude (Bessel functions and
+    phase in FP32, weight and products rounded), the sums add at most 12 roundings in a row,
+    and ez is twice its sum: 3e-6 S for the fields, 6e-6 S^2 for |ex|^2."""
+    rng = np.random.default_rng(n)
+    x, y, z = (rng.uniform(-2, 2, n).astype(np.float32) for _ in range(3))
+    x[0] = y[0] = 0.
+    if n > 8:
+        y[1] = 0.
+        z[2] = 0.
+        z[3:7] = 3e5, -3e5, 2e6, 1e5
+    res = bpm.focus_field_debye_at(x, y, z, .5, [.1, .7], 1.33, steps)
+    o = debye_ref.focus_field_debye_at(x, y, z, .5, [.1, .7], 1.33, steps)
+    zero = np.zeros(1, np.float32)
+    S = abs(debye_ref.focus_field_debye_at(zero, zero, zero, .5, [.1, .7], 1.33, steps)[1][0])
+    for v, b, k, tol in zip(res, o, ("u", "ex", "ey", "ez"), (6e-6 * S * S, 3e-6 * S, 3e-6 * S, 3e-6 * S)):
+        assert v.shape == b.shape and np.abs(v - b).max() < tol, k
+
+
 def test_variant_errors(bpm):
     with pytest.raises(NotImplementedError):
         bpm.focus_field_debye_gauss((2, 16, 16), (.1, .1, .1), .5, [0., .8])
