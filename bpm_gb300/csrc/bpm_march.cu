@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "fft_tile.cuh"
+#include "tcgen05.cuh"
 #include "warp_fft.cuh"
 
 using namespace bpmgb;
@@ -425,7 +426,7 @@ struct ColParams {
   int nx, ny, nz, z;         // z = step index: the field goes from plane z to z+1
   int prop_mode;             // 0 = table H, 1 = FP32 recipe with slice_n[z+1], 2 = weighted
   const float2* H;
-  const float2* Ht;          // H transposed (nx, ny), for the warp column kernels
+  const float2* Ht;          // H transposed (nx, ny): a column's entries are contiguous (cluster march)
   const float* kx2;
   const float* ky2;
   float k0f, dzf, n00f;
@@ -434,7 +435,7 @@ struct ColParams {
   const void* dn;            // weighted: dn of field 0 of the group (slice 0 is used)
   int dn_dtype;
   long long dn_bstride;
-  float* red_part;           // [G][ntiles][2]
+  float* red_part;           // weighted sums: [G][nx][2] per column (tile kernels [G][nx/16][2])
   float* dn0_field;          // [G]
   int scat;
   const float* sw;
@@ -512,19 +513,14 @@ __device__ __forceinline__ float2 plain_wave(const ColParams& p) {
 
 // k-space element (kx index x, ky index y) times the propagator, with the scattering partial
 // sums of bpm_3d.py:335-341 and the 1/(nx*ny) inverse-FFT normalisation folded in
-// COLUMN: the caller walks one column (x fixed, y over the lanes) and reads the transposed
-// table; ky2: the ky^2 table, in global or shared memory
-// htcol (COLUMN only, optional): the column's entries of the transposed table, staged
-template <bool COLUMN = false>
 __device__ __forceinline__ float2 prop_point(const ColParams& p, float2 v, int x, int y, float nk, float2 plain,
-                                             float& S, float& G, const float* ky2,
-                                             const float2* htcol = nullptr) {
+                                             float& S, float& G) {
   float2 h;
   if (p.prop_mode == 0) {
-    h = COLUMN ? (htcol ? htcol[y] : __ldg(p.Ht + (size_t)x * p.ny + y)) : __ldg(p.H + (size_t)y * p.nx + x);
+    h = __ldg(p.H + (size_t)y * p.nx + x);
     if (p.conj_h) h.y = -h.y;
   } else {
-    const float tmp = __fsub_rn(__fsub_rn(nk, __ldg(p.kx2 + x)), ky2[y]);
+    const float tmp = __fsub_rn(__fsub_rn(nk, __ldg(p.kx2 + x)), __ldg(p.ky2 + y));
     if (tmp >= 0.f) {
       const float ph = __fmul_rn(-p.dzf, __fsqrt_rn(tmp));
       sincosf(ph, &h.y, &h.x);
@@ -570,7 +566,7 @@ __device__ __forceinline__ void col_propagate(float2* tile, const ColParams& p, 
   for (int e = threadIdx.x; e < 16 * N; e += T) {
     const int y = e >> 4;
     const int c = e & 15;
-    tile[tile_idx(y, c)] = prop_point(p, tile[tile_idx(y, c)], x0 + c, y, nk, plain, S, G, p.ky2);
+    tile[tile_idx(y, c)] = prop_point(p, tile[tile_idx(y, c)], x0 + c, y, nk, plain, S, G);
   }
   if (p.scat) scat_partials_store<T>(p, S, G, gl, red);
   __syncthreads();
@@ -933,6 +929,47 @@ __global__ void grad_parts_sum_kernel(float* grad, const float* part, long long 
   grad[i] = sacc;
 }
 
+// Weighted-mode sums (sum |u| dn, sum |u|). Every kernel of the sequence-in-registers family
+// adds them in one order, so all give the same bits: a lane over its rows t, t + 32, ..., the
+// lanes of a column by this tree, and the columns by weighted_total.
+__device__ __forceinline__ float2 lane_tree2(float2 a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+  }
+  return a;
+}
+
+// dn0 = sum |u| dn / sum |u| (mult_dn_mean_buff, bpm_3d_kernels.cl:117) from the column sums
+// get(c), c < nx: lane t adds columns t, t + 32, ... (fetched U at a time), then the tree;
+// called by whole warps
+template <int U, class Get>
+__device__ __forceinline__ float weighted_total(int nx, int t, Get get) {
+  float2 a = make_float2(0.f, 0.f);
+  for (int c = t; c < nx; c += 32 * U) {
+    float2 v[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) v[k] = c + 32 * k < nx ? get(c + 32 * k) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      a.x += v[k].x;
+      a.y += v[k].y;
+    }
+  }
+  a = lane_tree2(a);
+  return a.x / a.y;
+}
+
+// the 16 column sums of a block of 512 threads in the coalesced tile mapping (r0, cc), from
+// the threads' sums over their rows: warp w ends up with column w's (all lanes). red: 16 x 33
+// float2 of shared memory that every thread is done reading.
+__device__ __forceinline__ float2 column_sums16(float sdn, float su, float2* red, int r0, int cc, int w, int t) {
+  red[cc * 33 + r0] = make_float2(sdn, su);
+  __syncthreads();
+  return lane_tree2(red[w * 33 + t]);
+}
+
 // Column pass without the tile transposition (128 <= N <= 1024, with or without scattering sums). The
 // block's 32*C threads load C columns (16, or 8 or 4 for small non-weighted passes) in the
 // coalesced tile mapping — thread (r0, cc) = (tid / C, tid % C) holds rows r0 + 32 i of column
@@ -941,9 +978,8 @@ __global__ void grad_parts_sum_kernel(float* grad, const float* part, long long 
 // first and last FFT stages run in it as well (colsplit_first / colsplit_last) and only the
 // middle stages per warp, on the column's exchange buffer. WHICH: 0 = forward FFT,
 // propagator, inverse FFT; 1 = forward FFT + weighted-mode partial sums (k-space stored back);
-// 2 = n from the partial sums, propagator, inverse FFT. The weighted passes keep C = 16: their
-// per-block partial sums then group the same elements in the same order as the cluster
-// kernel's.
+// 2 = n from the column sums, propagator, inverse FFT. The weighted passes keep C = 16: one
+// warp per column adds its sums.
 // Column buffers are STRIDE float2 apart: with 16 columns an odd stride puts a half-warp's
 // 16 columns on 16 different bank pairs; with 8 columns a half-warp spans two rows of 8
 // columns, conflict-free at N = 512 and 1024 for stride BUF + 2, 2-way on some accesses at
@@ -1084,19 +1120,10 @@ col_split_kernel(ColParams p) {
     for (int i = 0; i < E; i++) v[i] = Wp[gofs + i * gstep];
   }
   if (WHICH == 2 && warp == 0) {
-    // every block of the field sums the partials in index order, so all get the same n; the
-    // lanes fetch them at once (at most 64: nx <= 1024) and pass them on by shuffles
-    const int np = p.nx / 16;
-    const float* part = p.red_part + (size_t)gl * np * 2;
-    const float d0 = t < np ? part[2 * t] : 0.f, u0 = t < np ? part[2 * t + 1] : 0.f;
-    const float d1 = t + 32 < np ? part[2 * t + 64] : 0.f, u1 = t + 32 < np ? part[2 * t + 65] : 0.f;
-    float dn_sum = 0.f, u_sum = 0.f;
-    for (int i = 0; i < np; i++) {
-      dn_sum += __shfl_sync(0xffffffffu, i < 32 ? d0 : d1, i & 31);
-      u_sum += __shfl_sync(0xffffffffu, i < 32 ? u0 : u1, i & 31);
-    }
+    // every block of the field adds the column sums in the same order, so all get the same n
+    const float2* part = reinterpret_cast<const float2*>(p.red_part) + (size_t)gl * p.nx;
+    const float dn0 = weighted_total<16>(p.nx, t, [&](int c) { return part[c]; });
     if (t == 0) {
-      const float dn0 = dn_sum / u_sum;  // mult_dn_mean_buff, bpm_3d_kernels.cl:117
       s_n = p.n00f + dn0;                // mult_propagator_buff, bpm_3d_kernels.cl:482
       if (blockIdx.x == 0) p.dn0_field[gl] = dn0;
     }
@@ -1170,12 +1197,8 @@ col_split_kernel(ColParams p) {
         if (p.dn) sdn = fmaf(a, load_dn_real(p.dn, p.dn_dtype, gl * p.dn_bstride + k), sdn);
       }
     }
-    block_sum2<T>(sdn, su, red);
-    if (threadIdx.x == 0) {
-      float* o = p.red_part + ((size_t)gl * (p.nx / 16) + blockIdx.x) * 2;
-      o[0] = sdn;
-      o[1] = su;
-    }
+    const float2 cs = column_sums16(sdn, su, bufs, r0, cc, warp, t);
+    if (t == 0) reinterpret_cast<float2*>(p.red_part)[(size_t)gl * p.nx + x0 + warp] = cs;
   }
 }
 
@@ -1185,12 +1208,12 @@ col_split_kernel(ColParams p) {
 // column passes of the weighted mode (col_split_kernel<N, 1> and <N, 2>) become one kernel
 // whose blocks of a field form a thread-block cluster. A block is two 16-column tiles side
 // by side (two halves of 512 threads, each laid out and computing exactly as one block of
-// col_split_kernel: the same FFT stages, the same per-tile partial sums in the same order),
+// col_split_kernel: the same FFT stages, the same column sums in the same order),
 // so a field of nx / 16 tiles is a cluster of nx / 32 blocks (16 at nx = 512). Each half
-// stores its tile's two partials in shared memory; after a cluster barrier (a hardware
+// stores its tile's column sums in shared memory; after a cluster barrier (a hardware
 // barrier over blocks the launch co-schedules: no block waits on a block that has not
-// started), one warp per block reads all of the field's partials through distributed
-// shared memory in tile order and sums them as col_split_kernel<N, 2> does, so every block
+// started), one warp per block reads all of the field's column sums through distributed
+// shared memory and adds them as col_split_kernel<N, 2> does, so every block
 // gets the same n = n0 + dn0 bit for bit. The forward-transformed tile never leaves the
 // registers: propagator, inverse FFT and the coalesced store follow directly. A last
 // cluster barrier keeps each block's partials alive until every block has read them.
@@ -1220,8 +1243,7 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
   constexpr int TH = C * L;     // threads per half
   constexpr int T = Cfg::T;
   extern __shared__ __align__(16) float2 smem[];
-  __shared__ float red[2][32];
-  __shared__ float part[2][2];  // this block's two tile partials (sum |u| dn, sum |u|)
+  __shared__ float2 part[2 * C];  // this block's 32 column sums (sum |u| dn, sum |u|)
   __shared__ float s_n;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -1295,51 +1317,16 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
       if (p.dn) sdn = fmaf(a, load_dn_real(p.dn, p.dn_dtype, gl * p.dn_bstride + gofs + i * gstep), sdn);
     }
   }
-  // block_sum2<TH> of the half: warp trees, then the half's first thread over its warps in order
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    sdn += __shfl_xor_sync(0xffffffffu, sdn, o);
-    su += __shfl_xor_sync(0xffffffffu, su, o);
-  }
+  // (bufs: this half's column buffers, every thread past its last-stage reads)
   const int hw = ht >> 5;
-  if (t == 0) {
-    red[h][2 * hw] = sdn;
-    red[h][2 * hw + 1] = su;
-  }
-  __syncthreads();
-  if (ht == 0) {
-    float a = 0.f, b = 0.f;
-    for (int i = 0; i < TH / 32; i++) {
-      a += red[h][2 * i];
-      b += red[h][2 * i + 1];
-    }
-    part[h][0] = a;
-    part[h][1] = b;
-  }
-  cl.sync();  // every block's tile partials are visible across the cluster
+  const float2 cs = column_sums16(sdn, su, bufs, r0, cc, hw, t);
+  if (t == 0) part[h * C + hw] = cs;
+  cl.sync();  // every block's column sums are visible across the cluster
   if (warp == 0) {
-    // the field's partials in tile order (tile 2r + k in block rank r, half k), summed as
-    // col_split_kernel<N, 2> sums them
-    const int np = p.nx / 16;
-    float d0 = 0.f, u0 = 0.f, d1 = 0.f, u1 = 0.f;
-    if (t < np) {
-      const float* pr = cl.map_shared_rank(&part[0][0], t >> 1);
-      d0 = pr[2 * (t & 1)];
-      u0 = pr[2 * (t & 1) + 1];
-    }
-    if (t + 32 < np) {
-      const float* pr = cl.map_shared_rank(&part[0][0], (t + 32) >> 1);
-      d1 = pr[2 * (t & 1)];
-      u1 = pr[2 * (t & 1) + 1];
-    }
-    float dn_sum = 0.f, u_sum = 0.f;
-    for (int i = 0; i < np; i++) {
-      dn_sum += __shfl_sync(0xffffffffu, i < 32 ? d0 : d1, i & 31);
-      u_sum += __shfl_sync(0xffffffffu, i < 32 ? u0 : u1, i & 31);
-    }
+    // column c in block rank c / 32
+    const float dn0 = weighted_total<16>(p.nx, t, [&](int c) { return cl.map_shared_rank(part, c >> 5)[c & 31]; });
     if (t == 0) {
-      const float dn0 = dn_sum / u_sum;  // mult_dn_mean_buff, bpm_3d_kernels.cl:117
-      s_n = p.n00f + dn0;                // mult_propagator_buff, bpm_3d_kernels.cl:482
+      s_n = p.n00f + dn0;  // mult_propagator_buff, bpm_3d_kernels.cl:482
       if (blockIdx.x == 0) p.dn0_field[gl] = dn0;
     }
   }
@@ -1358,275 +1345,280 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
 }
 
 // ---------------------------------------------------------------------------------------
-// Whole-march cluster kernel for square grids N = 64, 128, 256: one thread-block cluster of
-// C = N/16 blocks per field (16 at 256, a non-portable cluster size) holds the field in
-// distributed shared memory for all nz steps. Block c owns rows [16c, 16c+16) (row slab R,
-// 16 x N) and columns [16c, 16c+16) (column slab K, N x 17 with one pad column). A step:
-// cluster barrier (row slabs ready) -> every block gathers its column slab from the other
-// blocks' row slabs through DSMEM (all remote loads of a batch issued before any store) ->
-// column FFT, [weighted: per-16-column-tile partial sums, exchanged through DSMEM after a
-// cluster barrier], propagator (the block's table columns and ky^2 staged once) -> inverse
-// column FFT -> cluster barrier (column slabs ready) -> every block gathers its row slab back
-// -> inverse row FFT, phase mask (the next plane's mask rows prefetched by cp.async during
-// the column pass), plane output, forward row FFT. The field never leaves the chip; one
-// launch runs the whole march of every field of the request. The FFTs, pointwise helpers and
-// the weighted partial sums (same 16-column tiles, same 512-thread element order, same
-// fixed-order total) are those of the pass kernels, so the results are the same bits (at
-// 64, where the pass kernels use the tile FFT, the same to FP32 rounding). Cluster barriers
-// are hardware barriers over blocks the launch co-schedules; a final barrier keeps every
-// block's shared memory alive until the others have finished reading it.
+// Whole-march cluster kernel for square grids N = 64, 128, 256: one thread-block cluster of C
+// blocks per field holds the field in shared memory and registers for all nz steps, in one
+// launch. Block c owns rows [S c, S c + S) in the row phases and columns [S c, S c + S) in the
+// column phases, one sequence of L lanes per row or column. A step:
+//   column phase: the column into registers, forward FFT, [weighted: the column's sums pushed
+//     to every block with st.async, the total from the N sums], propagator (the lane's entries
+//     of the table or ky^2 kept in registers for the whole march), inverse FFT;
+//   row phase: the row into registers, inverse FFT, phase mask (fetched during the column
+//     phase), plane output, forward FFT.
+// What bounds it is the chain of exchanges, not arithmetic or bandwidth: a field of 128^2 is 8
+// rows a block, so each phase ends as soon as the other blocks' data are there. Between the
+// phases every block sends one S x S tile to every block: the sequences write their values
+// transposed into C staged tiles (pitch S + 1, conflict-free both when a row is written and
+// when a column is read), and one cp.async.bulk per peer moves a tile into its shared memory
+// and counts it on its mbarrier. A block therefore waits for data, never for a cluster-wide
+// barrier: 0.44 us an exchange at 64^2 (8 blocks) and 0.68 us at 128^2 (16 blocks) measured
+// alone, against 1.2 us with st.async per element and a remote read round trip between two
+// cluster barriers before.
+// Buffers: a block that has all the tiles of an exchange knows that every peer had sent its
+// own, so had read the tiles of the exchange before; one buffer per direction is enough. The
+// staged tiles alternate between two buffers: when a block writes one again, the peers' tiles
+// of the exchange in between have arrived, which they sent after receiving the earlier ones.
+// The FFTs, pointwise helpers and the weighted sums are those of the pass kernels, so the
+// results are the same bits (at 64, where the pass kernels use the tile FFT, the same to FP32
+// rounding). Every wait is bounded in time; a block that gives up finishes the march without
+// further waits (its output is then wrong) and records it for bpm_device_status.
 // ---------------------------------------------------------------------------------------
-constexpr int kClusterThreads = 512;  // 16 warps
+constexpr unsigned long long kClusterWaitNs = 2000000000ull;  // a wait gives up after 2 s
+__device__ int g_march_status;                                // nonzero once a wait gave up
 
 struct ClusterArgs {
   RowParams rp;
   ColParams cp;
   const float2* u0;  // (batch, N, N)
   int nz;
-  int stage_mask;    // the next plane's mask (or dn) rows may be staged with 16-byte cp.async
+  unsigned long long wait_ns;
 };
 
 template <int N>
 struct ClusterCfg {
-  static constexpr int SLAB = 16;                  // rows (and columns) per block
-  static constexpr int C = N / SLAB;               // blocks per field (16 at 256: a non-portable size)
-  static constexpr int NW = kClusterThreads / 32;
-  static constexpr int TWPAD = (WarpFft<N>::TW + 1) & ~1;
-  static constexpr int KP = SLAB + 1;              // column-slab row pitch (float2)
-  static constexpr int GATHER = N * SLAB / kClusterThreads;  // slab elements per thread
-  // the next plane's mask rows and this block's propagator-table columns are staged in
-  // shared memory as well
-  static constexpr bool STAGE = true;
-  static constexpr size_t HT_F2 = STAGE ? (size_t)SLAB * N : 0;
-  static constexpr size_t MS_F2 = STAGE ? (size_t)SLAB * N : 0;  // up to 8 bytes per element
-  static constexpr size_t F2 = 2 * (size_t)TWPAD + (size_t)SLAB * N + (size_t)N * KP +
-                               (size_t)NW * WarpFft<N>::BUF + HT_F2 + MS_F2 + N / 2;
+  // lanes per sequence. 64 points on half-warps are three radix-4 stages with a warp for each
+  // scheduler of the SM (GB300, a weighted step: 2.98 us; on 8 lanes, two radix-8 stages but two
+  // warps a block, 3.76 us; half-warps in 16 blocks of 4 rows 3.33 us)
+  static constexpr int L = N == 64 ? 16 : 32;
+  static constexpr int E = N / L;
+  static constexpr int C = N == 64 ? 8 : 16;     // blocks per field (16: a non-portable cluster size)
+  static constexpr int S = N / C;                // rows (and columns) per block
+  static constexpr int T = S * L;                // threads
+  static constexpr int P = S + 1;                // tile row pitch (float2)
+  static constexpr int TS = S * P;               // tile (float2), a multiple of 16 bytes
+  static constexpr int EX = C * TS;              // one exchange buffer
+  static constexpr int TWPAD = (WarpFft<N, L>::TW + 1) & ~1;
+  static constexpr int BUF = WarpFft<N, L>::BUF;
+  // received tiles of the two directions, two staged sets, twiddles, FFT buffers, column sums
+  static constexpr size_t F2 = 4 * (size_t)EX + TWPAD + (size_t)S * BUF + N;
   static constexpr size_t SMEM = F2 * sizeof(float2);
-  static_assert(N * SLAB % kClusterThreads == 0 && SLAB % 16 == 0, "slab shape");
+  static_assert(TS % 2 == 0 && T >= C, "cluster shape");
 };
 
+// Waits for a phase of an mbarrier whose arrivals come from the cluster; once a wait of the
+// thread has given up (dead), further ones return at once.
+__device__ __forceinline__ void cluster_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, bool& dead) {
+  auto ready = [&] {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(tc::smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  if (dead || ready()) return;
+  const uint64_t t0 = tc::global_ns();
+  while (!ready())
+    if (tc::global_ns() - t0 > limit_ns) {
+      dead = true;
+      atomicExch(&g_march_status, 1);
+      return;
+    }
+}
+
+// the address of this block's shared-memory address a in the cluster's block r
+__device__ __forceinline__ uint32_t peer_addr(uint32_t a, uint32_t r) {
+  uint32_t o;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
+  return o;
+}
+
 template <int N>
-__global__ void __launch_bounds__(kClusterThreads, 1) cluster_march_kernel(ClusterArgs a) {
+__global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(ClusterArgs a) {
   namespace cg = cooperative_groups;
   using Cfg = ClusterCfg<N>;
-  constexpr int E = N / 32;
-  constexpr int T = kClusterThreads;
-  constexpr int NW = Cfg::NW;
-  constexpr int SLAB = Cfg::SLAB;
-  constexpr int KP = Cfg::KP;
-  constexpr int GA = Cfg::GATHER;
+  constexpr int L = Cfg::L, E = Cfg::E, S = Cfg::S, P = Cfg::P, TS = Cfg::TS, C = Cfg::C;
   cg::cluster_group cl = cg::this_cluster();
   const int c = (int)cl.block_rank();
-  const int gl = blockIdx.x / Cfg::C;
+  const int gl = blockIdx.x / C;
   const RowParams& p = a.rp;
   const ColParams& q = a.cp;
   extern __shared__ __align__(16) float2 csm[];
-  float2* twr = csm;
-  float2* twc = twr + Cfg::TWPAD;
-  float2* R = twc + Cfg::TWPAD;       // SLAB x N
-  float2* K = R + SLAB * N;           // N x KP
-  float2* X = K + (size_t)N * KP;     // NW exchange buffers
-  float2* HT = X + NW * WarpFft<N>::BUF;  // SLAB x N: propagator table columns (STAGE)
-  char* MS = reinterpret_cast<char*>(HT + Cfg::HT_F2);  // next plane's mask / dn rows (STAGE)
-  float* KY = reinterpret_cast<float*>(HT + Cfg::HT_F2 + Cfg::MS_F2);  // ky^2 (N floats)
-  __shared__ float red[64];
-  __shared__ float part[2 * (SLAB / 16)];  // this block's tile partials (weighted)
-  const int warp = threadIdx.x >> 5, t = threadIdx.x & 31;
-  float2* buf = X + warp * WarpFft<N>::BUF;
-  for (int k = threadIdx.x; k < WarpFft<N>::TW; k += T) {
-    twr[k] = p.wtw[k];
-    twc[k] = q.wtw[k];
-  }
-  for (int k = threadIdx.x; k < N; k += T) KY[k] = q.ky2[k];
-  const bool stage_ht = Cfg::STAGE && q.prop_mode == 0;
-  if (stage_ht)
-    for (int k = threadIdx.x; k < SLAB * N; k += T) HT[k] = q.Ht[(size_t)c * SLAB * N + k];
+  float2* K = csm;                    // received tiles: rows -> columns
+  float2* R = K + Cfg::EX;            // received tiles: columns -> rows
+  float2* stage0 = R + Cfg::EX;       // staged tiles, one set per direction
+  float2* tw = stage0 + 2 * Cfg::EX;
+  float2* sums = tw + Cfg::TWPAD + S * Cfg::BUF;  // weighted: the N column sums
+  __shared__ __align__(8) uint64_t bar[3];        // K, R and sums
+  const int tid = threadIdx.x, seq = tid / L, t = tid % L, lane = tid & 31;
+  float2* buf = tw + Cfg::TWPAD + seq * Cfg::BUF;
+  const int row = c * S + seq;        // this sequence's row, and its column
   const size_t plane = (size_t)N * N;
   const int nz = a.nz;
-  const bool stage_mask = Cfg::STAGE && a.stage_mask && p.do_mask;
-  const int mes = p.mask ? 8 : (p.dn_dtype == BPM_DN_C64 ? 8 : (p.dn_dtype == BPM_DN_F16 ? 2 : 4));
-  float dn0 = 0.f;  // weighted: dn0 of the last column pass
+  bool dead = false;
 
-  // the row pass producing plane z over this block's rows (z = 0: plane 0 is the input)
-  auto row_phase = [&](int z) {
-    const bool first = z == 0;
-    // the mean-index shift of plane z (row_dn0 of the pass kernels, whose p.z is the plane)
-    float dz0 = 0.f;
-    if (!first) {
-      if (p.mean_mode == BPM_MEAN_WEIGHTED)
-        dz0 = dn0;
-      else if (p.mean_mode == BPM_MEAN_SIMPLE && p.slice_dn0)
-        dz0 = p.slice_dn0[z];
+  if (tid == 0) {
+    for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
+    tc::fence_mbar_init();
+  }
+  for (int k = tid; k < WarpFft<N, L>::TW; k += Cfg::T) tw[k] = p.wtw[k];
+  // constants of the lane's column entries y = t + L m: the propagator table, or kx^2 and ky^2
+  // of the FP32 recipe, and dn slice 0 for the weighted sums
+  const bool table = q.prop_mode == 0, weighted = q.prop_mode == 2;
+  float2 hc[E];
+  float dnw[E];
+#pragma unroll
+  for (int m = 0; m < E; m++) {
+    const int y = t + L * m;
+    hc[m] = table ? q.Ht[(size_t)row * N + y] : make_float2(__ldg(q.ky2 + y), 0.f);
+    dnw[m] = (weighted && q.dn) ? load_dn_real(q.dn, q.dn_dtype, gl * q.dn_bstride + (size_t)y * N + row) : 0.f;
+  }
+  const float kx2 = __ldg(q.kx2 + row);
+  cl.sync();  // every block's mbarriers are initialised
+
+  // sends the sequence's values v[m] (element t + L m) to the blocks that own those elements
+  auto send = [&](const float2 (&v)[E], float2* dst, float2* stage, uint64_t* b) {
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      const int e = t + L * m;
+      stage[(e / S) * TS + (e % S) * P + seq] = v[m];
     }
-    const float2 rot = row_rot(p, dz0);
-    const size_t zoff = (size_t)z * plane;
-    for (int yl = warp; yl < SLAB; yl += NW) {
-      const int y = c * SLAB + yl;
-      float2 v[E];
-      if (first) {
-        const float2* src = a.u0 + gl * plane + (size_t)y * N;
-#pragma unroll
-        for (int m = 0; m < E; m++) v[m] = src[t + 32 * m];
-      } else {
-#pragma unroll
-        for (int m = 0; m < E; m++) v[m] = R[yl * N + t + 32 * m];
-        warp_fft<N, true>(v, buf, twr, t);
-      }
-      const char* mrow = MS + (size_t)yl * N * mes;
-#pragma unroll
-      for (int m = 0; m < E; m++) {
-        const int x = t + 32 * m;
-        const size_t pix = (size_t)y * N + x;
-        float2 u = v[m];
-        if (!first && p.do_mask) {
-          float2 M;
-          if (stage_mask) {
-            if (p.mask)
-              M = reinterpret_cast<const float2*>(mrow)[x];
-            else if (p.dn_dtype == BPM_DN_C64)
-              M = mask_from_complex(reinterpret_cast<const float2*>(mrow)[x], p.unit_k);
-            else
-              M = mask_from_real(p.dn_dtype == BPM_DN_F16 ? __half2float(reinterpret_cast<const __half*>(mrow)[x])
-                                                          : reinterpret_cast<const float*>(mrow)[x],
-                                 p.unit_k, x, y, p.nx, p.ny, p.absorb, p.taper);
-          } else {
-            M = p.mask ? p.mask[zoff + pix]
-                       : mask_value(p.dn, p.dn_dtype, gl * p.dn_bstride + zoff + pix, p.unit_k, x, y, p.nx, p.ny,
-                                    p.absorb, p.taper);
-          }
-          u = cmul(u, M);
-          if (dz0 != 0.f) u = cmul(u, rot);
-        }
-        if (p.out_kind == BPM_OUT_FIELD)
-          __stcs(reinterpret_cast<float2*>(p.out) + gl * p.out_bstride + zoff + pix, u);
-        else if (p.out_kind == BPM_OUT_INTENSITY)
-          __stcs(reinterpret_cast<float*>(p.out) + gl * p.out_bstride + zoff + pix, cabs2(u));
-        if (z == nz - 1 && p.last_plane) p.last_plane[gl * plane + pix] = u;
-        v[m] = u;
-      }
-      if (z + 1 < nz) {
-        warp_fft<N, false>(v, buf, twr, t);
-#pragma unroll
-        for (int m = 0; m < E; m++) R[yl * N + t + 32 * m] = v[m];
-      }
+    tc::fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) tc::mbar_expect_tx(b, (uint32_t)(Cfg::EX * sizeof(float2)));
+    if (tid < C) {
+      const int peer = (tid + c) % C;
+      asm volatile(
+          "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+              peer_addr(tc::smem_u32(dst + c * TS), peer)),
+          "r"(tc::smem_u32(stage + peer * TS)), "r"((uint32_t)(TS * sizeof(float2))),
+          "r"(peer_addr(tc::smem_u32(b), peer))
+          : "memory");
     }
   };
+  auto receive = [&](float2 (&v)[E], const float2* src) {
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+      const int e = t + L * m;
+      v[m] = src[(e / S) * TS + seq * P + e % S];
+    }
+  };
+  auto store_plane = [&](int z, int m, float2 u) {
+    const size_t pix = (size_t)row * N + t + L * m, o = (size_t)z * plane + pix;
+    if (p.out_kind == BPM_OUT_FIELD)
+      __stcs(reinterpret_cast<float2*>(p.out) + gl * p.out_bstride + o, u);
+    else if (p.out_kind == BPM_OUT_INTENSITY)
+      __stcs(reinterpret_cast<float*>(p.out) + gl * p.out_bstride + o, cabs2(u));
+    if (z == nz - 1 && p.last_plane) p.last_plane[gl * plane + pix] = u;
+  };
 
-  __syncthreads();  // tables
-  row_phase(0);
-  for (int i = 0; i + 1 < nz; i++) {
-    cl.sync();  // every row slab holds the row-transformed field
-    {
-      // gather the column slab K[y][xl] = R_{y/SLAB}[y%SLAB][SLAB c + xl]: all remote loads
-      // first, then the stores
-      float2 g[GA];
+  float2 v[E];
 #pragma unroll
-      for (int k = 0; k < GA; k++) {
-        const int e = threadIdx.x + k * T;
-        const int y = e / SLAB, xl = e % SLAB;
-        const float2* Rr = cl.map_shared_rank(R, y / SLAB);
-        g[k] = Rr[(y % SLAB) * N + c * SLAB + xl];
-      }
+  for (int m = 0; m < E; m++) v[m] = a.u0[gl * plane + (size_t)row * N + t + L * m];
 #pragma unroll
-      for (int k = 0; k < GA; k++) {
-        const int e = threadIdx.x + k * T;
-        K[(e / SLAB) * KP + e % SLAB] = g[k];
+  for (int m = 0; m < E; m++) store_plane(0, m, v[m]);
+  if (nz > 1) {
+    warp_fft<N, false, L>(v, buf, tw, t);
+    send(v, K, stage0, &bar[0]);
+  }
+  for (int z = 1; z < nz; z++) {
+    const uint32_t ph = (uint32_t)(z - 1) & 1u;
+    // the row's mask (or dn) values of plane z, used in the row phase
+    float2 mk[E];
+    if (p.do_mask) {
+      const size_t off = (size_t)z * plane + (size_t)row * N + t;
+#pragma unroll
+      for (int m = 0; m < E; m++) {
+        if (p.mask)
+          mk[m] = p.mask[off + L * m];
+        else if (p.dn_dtype == BPM_DN_C64)
+          mk[m] = __ldg(reinterpret_cast<const float2*>(p.dn) + gl * p.dn_bstride + off + L * m);
+        else
+          mk[m].x = load_dn_real(p.dn, p.dn_dtype, gl * p.dn_bstride + off + L * m);
       }
     }
-    if (stage_mask) {
-      // the rows of plane i+1's mask (or dn) this block will apply, fetched during the
-      // column pass
-      const size_t off = (size_t)(i + 1) * plane + (size_t)c * SLAB * N;
-      const char* src = p.mask ? reinterpret_cast<const char*>(p.mask + off)
-                               : static_cast<const char*>(p.dn) + ((size_t)gl * p.dn_bstride + off) * mes;
-      for (int o = threadIdx.x * 16; o < SLAB * N * mes; o += T * 16) cp_async16(MS + o, src + o);
-      cp_async_commit();
-    }
-    __syncthreads();
-    float n_eff = q.prop_mode == 1 ? q.slice_n[i + 1] : q.n00f;
-    if (q.prop_mode == 2) {
-      // weighted: forward transforms, k-space back into the slab, tile partial sums
-      for (int xl = warp; xl < SLAB; xl += NW) {
-        float2 v[E];
+    float n_eff = q.prop_mode == 1 ? q.slice_n[z] : q.n00f;
+    float dn0 = (p.mean_mode == BPM_MEAN_SIMPLE && p.slice_dn0) ? p.slice_dn0[z] : 0.f;
+
+    // ---- column phase ----
+    cluster_wait(&bar[0], ph, a.wait_ns, dead);
+    receive(v, K);
+    warp_fft<N, false, L>(v, buf, tw, t);
+    if (weighted) {
+      float2 sm = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int m = 0; m < E; m++) v[m] = K[(t + 32 * m) * KP + xl];
-        warp_fft<N, false>(v, buf, twc, t);
+      for (int m = 0; m < E; m++) {
+        const float aa = __fsqrt_rn(cabs2(v[m]));
+        sm.y += aa;
+        sm.x = fmaf(aa, dnw[m], sm.x);
+      }
 #pragma unroll
-        for (int m = 0; m < E; m++) K[(t + 32 * m) * KP + xl] = v[m];
+      for (int o = L / 2; o > 0; o >>= 1) {
+        sm.x += __shfl_xor_sync(0xffffffffu, sm.x, o);
+        sm.y += __shfl_xor_sync(0xffffffffu, sm.y, o);
       }
-      __syncthreads();
-      constexpr int PER = 16 * N / T;  // the warp kernels' element order within a tile
-      for (int tile = 0; tile < SLAB / 16; tile++) {
-        const int x0 = c * SLAB + tile * 16;
-        float sdn = 0.f, su = 0.f;
-#pragma unroll
-        for (int ii = 0; ii < PER; ii++) {
-          const int e = threadIdx.x + ii * T;
-          const int n = e >> 4, cc = e & 15;
-          const float2 u = K[n * KP + tile * 16 + cc];
-          const float aa = __fsqrt_rn(cabs2(u));
-          su += aa;
-          if (q.dn)
-            sdn = fmaf(aa, load_dn_real(q.dn, q.dn_dtype, gl * q.dn_bstride + (size_t)n * N + x0 + cc), sdn);
-        }
-        block_sum2<T>(sdn, su, red);
-        if (threadIdx.x == 0) {
-          part[2 * tile] = sdn;
-          part[2 * tile + 1] = su;
-        }
-        __syncthreads();
-      }
-      cl.sync();  // every block's partials are visible
-      if (threadIdx.x == 0) {
-        float dn_sum = 0.f, u_sum = 0.f;
-        for (int r = 0; r < Cfg::C; r++) {
-          const float* pr = cl.map_shared_rank(part, r);
-          for (int tile = 0; tile < SLAB / 16; tile++) {
-            dn_sum += pr[2 * tile];
-            u_sum += pr[2 * tile + 1];
-          }
-        }
-        red[0] = dn_sum / u_sum;  // mult_dn_mean_buff, bpm_3d_kernels.cl:117
-      }
-      __syncthreads();
-      dn0 = red[0];
+      if (tid == 0) tc::mbar_expect_tx(&bar[2], (uint32_t)(N * sizeof(float2)));
+      for (int r = t; r < C; r += L)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(
+                         peer_addr(tc::smem_u32(sums + row), r)),
+                     "f"(sm.x), "f"(sm.y), "r"(peer_addr(tc::smem_u32(&bar[2]), r))
+                     : "memory");
+      cluster_wait(&bar[2], ph, a.wait_ns, dead);
+      __syncwarp();
+      dn0 = weighted_total<N / 32>(N, lane, [&](int i) { return sums[i]; });
       n_eff = q.n00f + dn0;  // mult_propagator_buff, bpm_3d_kernels.cl:482
     }
-    const float nk = prop_nk(q, n_eff);
-    for (int xl = warp; xl < SLAB; xl += NW) {
-      const int x = c * SLAB + xl;
-      float2 v[E];
+    const float nkx = table ? 0.f : __fsub_rn(prop_nk(q, n_eff), kx2);
 #pragma unroll
-      for (int m = 0; m < E; m++) v[m] = K[(t + 32 * m) * KP + xl];
-      if (q.prop_mode != 2) warp_fft<N, false>(v, buf, twc, t);
-      float S = 0.f, G = 0.f;
-      const float2* htc = stage_ht ? HT + (size_t)xl * N : nullptr;
+    for (int m = 0; m < E; m++) {
+      float2 h = hc[m];
+      if (!table) {
+        const float tmp = __fsub_rn(nkx, hc[m].x);
+        h = make_float2(0.f, 0.f);
+        if (tmp >= 0.f) sincosf(__fmul_rn(-q.dzf, __fsqrt_rn(tmp)), &h.y, &h.x);
+      }
+      v[m] = cscale(cmul(v[m], h), q.scale);
+    }
+    warp_fft<N, true, L>(v, buf, tw, t);
+    send(v, R, stage0 + Cfg::EX, &bar[1]);
+
+    // ---- row phase ----
+    const float2 rot = row_rot(p, dn0);
+    if (p.do_mask && !p.mask) {
 #pragma unroll
       for (int m = 0; m < E; m++)
-        v[m] = prop_point<true>(q, v[m], x, t + 32 * m, nk, make_float2(0.f, 0.f), S, G, KY, htc);
-      warp_fft<N, true>(v, buf, twc, t);
-#pragma unroll
-      for (int m = 0; m < E; m++) K[(t + 32 * m) * KP + xl] = v[m];
+        mk[m] = p.dn_dtype == BPM_DN_C64
+                    ? mask_from_complex(mk[m], p.unit_k)
+                    : mask_from_real(mk[m].x, p.unit_k, t + L * m, row, N, N, p.absorb, p.taper);
     }
-    cl.sync();  // every column slab holds the propagated field
-    {
-      // gather the row slab back: R[yl][x] = K_{x/SLAB}[SLAB c + yl][x%SLAB]
-      float2 g[GA];
+    cluster_wait(&bar[1], ph, a.wait_ns, dead);
+    receive(v, R);
+    warp_fft<N, true, L>(v, buf, tw, t);
+    if (p.do_mask) {
 #pragma unroll
-      for (int k = 0; k < GA; k++) {
-        const int e = threadIdx.x + k * T;
-        const int yl = e / N, x = e % N;
-        const float2* Kr = cl.map_shared_rank(K, x / SLAB);
-        g[k] = Kr[(c * SLAB + yl) * KP + x % SLAB];
+      for (int m = 0; m < E; m++) {
+        v[m] = cmul(v[m], mk[m]);
+        if (dn0 != 0.f) v[m] = cmul(v[m], rot);
       }
-#pragma unroll
-      for (int k = 0; k < GA; k++) R[threadIdx.x + k * T] = g[k];
     }
-    if (stage_mask) cp_async_wait<0>();  // this thread's pieces of the next plane's mask rows
-    __syncthreads();
-    row_phase(i + 1);
+    float2 u[E];
+#pragma unroll
+    for (int m = 0; m < E; m++) u[m] = v[m];
+    if (z + 1 < nz) {
+      warp_fft<N, false, L>(v, buf, tw, t);
+      send(v, K, stage0, &bar[0]);
+    }
+#pragma unroll
+    for (int m = 0; m < E; m++) store_plane(z, m, u[m]);  // after the tiles are on their way
   }
-  cl.sync();  // no block leaves while another may still read its slabs
+  if (dead) {  // copies that were late still land before any block of the cluster leaves
+    const uint64_t t0 = tc::global_ns();
+    while (tc::global_ns() - t0 < 5000000ull) {
+    }
+  }
+  cl.sync();  // no block leaves while its tiles are being read or another may still send to it
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1664,24 +1656,6 @@ int sm_count() {
     return v > 0 ? v : 1;
   }();
   return n;
-}
-
-// blocks of `kernel` resident on the whole device at once
-template <class Kern>
-int resident_blocks(Kern kernel, int threads, size_t smem) {
-  int dev = 0, nsm = 1, occ = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
-  cudaGetLastError();
-  return std::max(1, occ) * std::max(1, nsm);
-}
-
-// workers for `items` work items with at most `cap` workers, every worker taking the same
-// number of items (the last one possibly fewer)
-inline int balanced_workers(int items, int cap) {
-  const int per = (items + cap - 1) / cap;
-  return (items + per - 1) / per;
 }
 
 template <int N>
@@ -2025,7 +1999,7 @@ WsLayout ws_layout(const bpm_plan* pl, int G) {
   L.w = off;
   off += align256((size_t)G * pl->d.nx * pl->d.ny * sizeof(float2));
   L.red = off;
-  off += align256((size_t)G * ntiles * 2 * sizeof(float));
+  off += align256((size_t)G * pl->d.nx * sizeof(float2));
   L.dn0 = off;
   off += align256((size_t)G * sizeof(float));
   L.scat = off;
@@ -2282,23 +2256,30 @@ int sink_copy(bpm_plan* pl, const bpm_request* r, const HostSink& h, int b0, int
   return BPM_OK;
 }
 
-// The whole-march cluster kernel serves square grids without scattering sums or
-// checkpoints. Measured on GB300, one field: at 64^2 it beats the pass kernels (Nz 64
-// weighted 0.40 vs 0.82 ms); at 128^2 the pass kernels are faster since a single field's row
-// pass stages its mask row (Nz 128 weighted 1.08 vs 1.14 ms, ignore 0.59 vs 0.81 ms, the
-// same bits), and at 256^2 too (Nz 256 ignore 1.47 vs 2.70 ms). So by default it takes
-// N = 64; BPM_GB300_CLUSTER=1 extends it to 128 and 256, =0 turns it off, and a side
-// length (64, 128 or 256) makes it the default up to that side.
-bool cluster_enabled(int n) {
+// The whole-march cluster kernel serves square grids of 64, 128 and 256 without scattering sums
+// or checkpoints. Where it is the default (GB300, us per step, cluster kernel against the pass
+// kernels of the same march replayed as a graph):
+//   64^2: always (1 field weighted 3.0 against 11.7, 64 fields 4.5 against 14.0);
+//   128^2: the weighted mode (1 field 4.2 against 7.6, 12 fields 5.5 against 9.2, 64 fields 19.2
+//     against 21.1) and up to 32 fields otherwise (1 field 3.1 against 4.1, 32 fields 8.7 against
+//     9.5; 64 fields 16.8 against 16.4);
+//   256^2: the weighted mode up to 4 fields (8.8 against 9.6 for 1 field and 11.0 for 4); a field
+//     fills 16 SMs there, so 8 fields take 17.6 against 12.4, and without the sums one field
+//     6.7 against 4.8.
+// BPM_GB300_CLUSTER=1 takes it wherever it serves, =0 nowhere, and a side length (64, 128 or
+// 256) wherever it serves up to that side.
+bool cluster_default(int n, int mean_mode, int batch) {
   static const int max_side = [] {
     const char* e = getenv("BPM_GB300_CLUSTER");
-    if (!e) return 64;
+    if (!e) return -1;
     if (strcmp(e, "0") == 0) return 0;
     if (strcmp(e, "1") == 0) return 256;
     const int v = atoi(e);
     return v >= 64 ? v : 64;
   }();
-  return n <= max_side;
+  if (max_side >= 0) return n <= max_side;
+  const bool weighted = mean_mode == BPM_MEAN_WEIGHTED;
+  return n == 64 || (n == 128 && (weighted || batch <= 32)) || (n == 256 && weighted && batch <= 4);
 }
 
 template <int N>
@@ -2307,7 +2288,7 @@ struct ClusterK {
     using Cfg = ClusterCfg<N>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(batch * Cfg::C);
-    cfg.blockDim = dim3(kClusterThreads);
+    cfg.blockDim = dim3(Cfg::T);
     cfg.dynamicSmemBytes = Cfg::SMEM;
     cfg.stream = s;
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2345,11 +2326,7 @@ struct ClusterK {
     a.cp = c.cp;
     a.u0 = static_cast<const float2*>(r->u0);
     a.nz = pl->d.nz;
-    {
-      const int es = r->mask ? 8 : (r->dn_dtype == BPM_DN_C64 ? 8 : (r->dn_dtype == BPM_DN_F16 ? 2 : 4));
-      a.stage_mask = r->mask ? aligned16(r->mask)
-                             : (aligned16(r->dn) && ((size_t)r->dn_batch_stride * es) % 16 == 0);
-    }
+    a.wait_ns = kClusterWaitNs;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = config((unsigned)r->batch, s, at);
     BPM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_march_kernel<N>, a));
@@ -2362,7 +2339,7 @@ struct ClusterK {
 constexpr int kNotCluster = 1;
 int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
   const bpm_grid_desc& d = pl->d;
-  const bool want = r->cluster == 1 || (r->cluster == 0 && cluster_enabled(d.nx));
+  const bool want = r->cluster == 1 || (r->cluster == 0 && cluster_default(d.nx, d.mean_mode, r->batch));
   if (d.nx != d.ny || !want || r->scatter_p || r->ckpt || !pl->wtw_x || !pl->wtw_y) return kNotCluster;
   switch (d.nx) {
     case 64: return ClusterK<64>::ready() ? ClusterK<64>::launch(pl, r, ws, s) : kNotCluster;
@@ -2626,6 +2603,15 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
 
 }  // namespace
 
+int bpmgb::march_status(int clear, int* v) {
+  BPM_CUDA_TRY(cudaMemcpyFromSymbol(v, g_march_status, sizeof(int)));
+  if (clear && *v) {
+    const int zero = 0;
+    BPM_CUDA_TRY(cudaMemcpyToSymbol(g_march_status, &zero, sizeof(int)));
+  }
+  return BPM_OK;
+}
+
 // ---------------------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------------------
@@ -2730,7 +2716,7 @@ extern "C" int bpm_plan_create(const bpm_grid_desc* d, bpm_plan** out) {
   for (int axis = 0; axis < 2; axis++) {
     const int n = axis == 0 ? nx : ny;
     if (n < 64 || n > 1024) continue;  // the warp FFT's sizes (the cluster kernel uses 64 too)
-    std::vector<float2> w = warp_twiddles(n);
+    std::vector<float2> w = warp_twiddles(n, n == 64 ? ClusterCfg<64>::L : 32);
     float2** dst = axis == 0 ? &pl->wtw_x : &pl->wtw_y;
     if ((e = cudaMalloc(dst, w.size() * sizeof(float2)))) return fail(e, "cudaMalloc");
     if ((e = cudaMemcpy(*dst, w.data(), w.size() * sizeof(float2), cudaMemcpyHostToDevice)))

@@ -19,6 +19,10 @@ void set_error(const std::string& msg);
 void clear_error();
 int cuda_fail(cudaError_t e, const char* what);
 
+// sticky status of the marches' bounded waits (nonzero once one gave up), read from the
+// current device and cleared on request; BPM_OK or a negative status
+int march_status(int clear, int* v);
+
 // number of kernels launched by this library (bpm_launch_count)
 extern std::atomic<unsigned long long> g_launches;
 inline void count_launch(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }

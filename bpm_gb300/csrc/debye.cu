@@ -1577,7 +1577,9 @@ extern "C" int bpm_device_status(int clear) {
     const int zero = 0;
     BPM_CUDA_TRY(cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(int)));
   }
-  return v;
+  int m = 0;
+  const int rc = march_status(clear, &m);
+  return rc != BPM_OK ? rc : (v | m);
 }
 
 // Self-test of the bounded waits of debye_accum_tc_kernel: one block on a small product whose

@@ -534,3 +534,29 @@ def test_cluster_march_matches_pass_kernels(bpm, tmp_path):
         elif not np.array_equal(A[k], B[k]):
             bad.append((k, rel_l2(A[k], B[k])))
     assert not bad, bad
+
+
+@pytest.mark.parametrize("side,mode,kind,batch", [(128, "ignore", "c64", 33), (128, "ignore", "f32", 32),
+                                                  (256, "weighted", "f16", 4), (256, "weighted", "f32", 5),
+                                                  (64, "simple", "f16", 70), (64, "weighted", "none", 1)])
+def test_cluster_rule_does_not_change_a_result(bpm, side, mode, kind, batch):
+    """Either side of the batch sizes at which a square grid changes between the whole-march
+    cluster kernel and the pass kernels: each field of the batch equals the field marched
+    alone bit for bit, and the FP64 oracle to the parity tolerance."""
+    nz = 5
+    rng = np.random.default_rng(batch)
+    dn = None
+    if kind != "none":
+        dn = (.03 * rng.standard_normal((nz, side, side))).astype(np.float32)
+        if kind == "c64":
+            dn = (dn - 1j * np.abs(.002 * rng.standard_normal(dn.shape))).astype(np.complex64)
+    x = .1 * np.arange(side)
+    u0 = np.exp(2j * np.pi * rng.uniform(-.3, .3, (batch, 1, 1)) * x[None, None, :]).repeat(side, 1).astype(np.complex64)
+    kw = dict(lam=.5, n0=1.33, dn=dn, mean_mode=mode, absorbing_width=4, store_dn_as_half=kind == "f16")
+    ub = bpm.bpm_3d_batched((side, side, nz), (.1, .1, .1), u0=u0, **kw)
+    for b in sorted({0, batch // 2, batch - 1}):
+        us = bpm.bpm_3d((side, side, nz), (.1, .1, .1), u0=u0[b], **kw)
+        assert np.array_equal(ub[b], us), b
+        o = bpm_ref.bpm_3d((side, side, nz), (.1, .1, .1), u0=u0[b], precision="fp64", **kw)
+        assert rel_l2(us, o) < TOL, b
+    assert bpm._native.lib().bpm_device_status(0) == 0
