@@ -666,7 +666,9 @@ class MixedBatch:
             shape = (B, Nz, Ny, Nx)
             out = torch.empty(shape, dtype=torch.complex64 if ok == N.OUT_FIELD else torch.float32, device=dev)
             last = torch.empty((B, Ny, Nx), dtype=torch.complex64, device=dev)
-            launch = {}
+            # groups march beside one another: pass kernels, which interleave (the one-launch
+            # march of a few fields would hold its part of every SM until it ends)
+            launch = {"cluster": 2} if len(groups) > 1 and min(Nx, Ny) >= 128 and (Nx, Ny) != (128, 128) else {}
             if tune:
                 from .autotune import tune_shape
                 launch = tune_shape((Nx, Ny, Nz), r0.units, r0.lam, r0.n0, B, dn, r0.mean_mode, out_kind,

@@ -33,6 +33,8 @@
 
 #include "common.cuh"
 #include "fft_tile.cuh"
+#include "march.cuh"
+#include "march_grid.cuh"
 #include "tcgen05.cuh"
 #include "warp_fft.cuh"
 
@@ -173,113 +175,10 @@ __global__ void build_tables_kernel(int nx, int ny, double dx, double dy, double
 // ---------------------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------------------
-struct RowParams {
-  const float2* src;        // group's input planes (u0 + b0*plane, or W)
-  long long src_bstride;    // float2 elements between fields
-  float2* W;                // group workspace planes
-  int nx, ny, nz, z;        // z = plane produced by this pass (dn slice index)
-  int do_inv, do_fwd, do_mask;
-  const void* dn;           // dn of field 0 of the group
-  int dn_dtype;
-  long long dn_bstride;     // elements
-  float unit_k;
-  int absorb;
-  const float* taper;
-  int mean_mode;
-  const float* dn0_field;   // weighted: per group field
-  const float* slice_dn0;   // simple: per slice
-  void* out;                // output of field 0 of the group
-  int out_kind;
-  long long out_bstride;    // elements
-  int zout0;                // output plane index = z - zout0
-  float2* last_plane;       // group's exit planes or NULL
-  float2* ckpt;             // group's checkpoint planes (G, n_ckpt, ny, nx) or NULL
-  int ckpt_every, n_ckpt;
-  const float* scat_part;   // [G][ntiles][2]
-  int n_ctiles;
-  float* scat_p;            // group's (nz) rows
-  float* scat_g;
-  float prefac_f;
-  const float2* tw;
-  const float2* wtw;        // stage-ordered twiddles of the warp FFT
-  // adjoint passes only
-  const float2* seg;        // forward fields of the current segment (G, planes, ny, nx)
-  long long seg_bstride;    // float2 elements between fields
-  int seg_z0;               // plane index of the segment's first plane
-  float* grad_dn;           // group's (nz, ny, nx) dn gradients
-  float2* grad_u0;          // group's (ny, nx) u0 gradients or NULL
-  const float2* mask;       // precomputed masks of the shared dn, (nz, ny, nx), or NULL
-  // adjoint with the dn gradient summed over the fields (row_adj_shared_kernel, grad_sum 1):
-  // block 0 of a row writes its fields' sum to grad_dn, block b >= 1 to grad_part + (b - 1) *
-  // grad_part_stride, stored (grad_acc 0, the first group of the request) or added (grad_acc
-  // 1, the later groups)
-  int grad_sum;
-  float* grad_part;
-  long long grad_part_stride;
-  int grad_acc;
-};
-
-__device__ __forceinline__ float load_dn_real(const void* dn, int dtype, size_t idx) {
-  if (dtype == BPM_DN_F16) return __half2float(reinterpret_cast<const __half*>(dn)[idx]);
-  return __ldg(reinterpret_cast<const float*>(dn) + idx);
-}
-
 // The pointwise work of a row pass on one element v = u(x, y) of plane z, shared by the
 // tile and warp row kernels. Forward: phase mask of dn slice z (+ taper) and the plane-z
 // outputs. Adjoint: dn gradient against the forward field, conjugate mask; at plane 0 the
 // adjoint value is the u0 gradient.
-// Phase mask of dn slice z at (x, y): M = taper * exp(-i k0 dz dn) for real dn
-// (mult_dn*, bpm_3d_kernels.cl:20-81, 198-262), exp(k0 dz Im dn) * exp(-i k0 dz Re dn) with
-// no taper for complex dn (mult_dn*_complex, :84-101, :265-283). The mean-index shift dn0
-// enters as the separate factor exp(+i k0 dz dn0) (row_rot), so M depends on dn alone and
-// can be computed once per dn volume for a whole batch (bpm_mask_precompute); the on-the-fly
-// and precomputed masks are the same FP32 arithmetic, bit for bit.
-__device__ __forceinline__ float2 mask_from_complex(float2 d, float unit_k) {
-  float s, c;
-  const float m = expf(unit_k * d.y);
-  sincosf((-unit_k) * d.x, &s, &c);
-  return make_float2(m * c, m * s);
-}
-
-__device__ __forceinline__ float2 mask_from_real(float dnv, float unit_k, int x, int y, int nx, int ny, int absorb,
-                                                 const float* taper) {
-  float s, c;
-  sincosf((-unit_k) * dnv, &s, &c);
-  float2 M = make_float2(c, s);
-  const int dist = min(min(nx - 1 - x, x), min(ny - 1 - y, y));
-  if (dist < absorb) {
-    const float a = taper[dist];
-    M.x *= a;
-    M.y *= a;
-  }
-  return M;
-}
-
-__device__ __forceinline__ float2 mask_value(const void* dn, int dtype, size_t idx, float unit_k, int x, int y,
-                                             int nx, int ny, int absorb, const float* taper) {
-  if (dtype == BPM_DN_C64) return mask_from_complex(__ldg(reinterpret_cast<const float2*>(dn) + idx), unit_k);
-  return mask_from_real(load_dn_real(dn, dtype, idx), unit_k, x, y, nx, ny, absorb, taper);
-}
-
-// PRE = 1: the masks come precomputed (p.mask); PRE = 0: formed on the fly from dn. The
-// two are compiled separately so the precomputed kernel carries no sincosf.
-template <int PRE>
-__device__ __forceinline__ float2 row_mask(const RowParams& p, int x, int y, int gl, size_t zoff, size_t pix) {
-  if constexpr (PRE == 1) {
-    return p.mask[zoff + pix];
-  } else {
-    return mask_value(p.dn, p.dn_dtype, gl * p.dn_bstride + zoff + pix, p.unit_k, x, y, p.nx, p.ny, p.absorb,
-                      p.taper);
-  }
-}
-
-// exp(+i k0 dz dn0), the mean-index shift of the mask (identity when dn0 = 0)
-__device__ __forceinline__ float2 row_rot(const RowParams& p, float dn0) {
-  float s, c;
-  sincosf(p.unit_k * dn0, &s, &c);
-  return make_float2(c, s);
-}
-
 template <bool ADJ, int PRE>
 __device__ __forceinline__ float2 row_point(const RowParams& p, float2 v, int x, int y, int gl, size_t plane,
                                             size_t zoff, size_t ooff, float dn0, float2 rot, bool last,
@@ -421,61 +320,6 @@ row_pass_kernel(RowParams p) {
   }
 }
 
-struct ColParams {
-  float2* W;
-  int nx, ny, nz, z;         // z = step index: the field goes from plane z to z+1
-  int prop_mode;             // 0 = table H, 1 = FP32 recipe with slice_n[z+1], 2 = weighted
-  const float2* H;
-  const float2* Ht;          // H transposed (nx, ny): a column's entries are contiguous (cluster march)
-  const float* kx2;
-  const float* ky2;
-  float k0f, dzf, n00f;
-  const float* slice_n;
-  float scale;               // 1/(nx*ny)
-  const void* dn;            // weighted: dn of field 0 of the group (slice 0 is used)
-  int dn_dtype;
-  long long dn_bstride;
-  float* red_part;           // weighted sums: [G][nx][2] per column (tile kernels [G][nx/16][2])
-  float* dn0_field;          // [G]
-  int scat;
-  const float* sw;
-  const float* gw;
-  float* scat_part;          // [G][ntiles][2]
-  double plain_phase;        // k0*n0*dz
-  int spi;                   // scattering_plane_ind
-  int conj_h;                // adjoint: multiply by conj(H)
-  const float2* tw;
-  const float2* wtw;         // stage-ordered twiddles of the warp FFT
-  int dn_stage;              // weighted: dn rows may be staged with 16-byte cp.async
-  int col_block;             // 0: the library's rule; 4, 8 or 16 columns per non-weighted block
-  int col_fuse;              // weighted: 1 one fused column pass where available, 0 or 2 two passes
-};
-
-template <int T>
-__device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  constexpr int NW = (T + 31) / 32;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    red[2 * w] = a;
-    red[2 * w + 1] = b;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.f, t = 0.f;
-    for (int i = 0; i < NW; i++) {
-      s += red[2 * i];
-      t += red[2 * i + 1];
-    }
-    a = s;
-    b = t;
-  }
-}
-
 template <int N, int T = TileCfg<N>::THREADS>
 __device__ __forceinline__ void col_load(float2* tile, const float2* Wp, int nx, int x0) {
   constexpr int PER = 16 * N / T;
@@ -502,15 +346,6 @@ __device__ __forceinline__ void col_store(const float2* tile, float2* Wp, int nx
   }
 }
 
-// plain_wave_dct[z+1] = nx*ny*exp(-i k0 n0 (spi + z+1) dz) of bpm_3d.py:253, FP64 then complex64
-__device__ __forceinline__ float2 plain_wave(const ColParams& p) {
-  double ph = -p.plain_phase * (double)(p.spi + p.z + 1);
-  double s, c;
-  sincos(ph, &s, &c);
-  double m = (double)p.nx * (double)p.ny;
-  return make_float2((float)(m * c), (float)(m * s));
-}
-
 // k-space element (kx index x, ky index y) times the propagator, with the scattering partial
 // sums of bpm_3d.py:335-341 and the 1/(nx*ny) inverse-FFT normalisation folded in
 __device__ __forceinline__ float2 prop_point(const ColParams& p, float2 v, int x, int y, float nk, float2 plain,
@@ -521,12 +356,7 @@ __device__ __forceinline__ float2 prop_point(const ColParams& p, float2 v, int x
     if (p.conj_h) h.y = -h.y;
   } else {
     const float tmp = __fsub_rn(__fsub_rn(nk, __ldg(p.kx2 + x)), __ldg(p.ky2 + y));
-    if (tmp >= 0.f) {
-      const float ph = __fmul_rn(-p.dzf, __fsqrt_rn(tmp));
-      sincosf(ph, &h.y, &h.x);
-    } else {
-      h = make_float2(0.f, 0.f);
-    }
+    h = tmp >= 0.f ? cos_sin(__fmul_rn(-p.dzf, __fsqrt_rn(tmp))) : make_float2(0.f, 0.f);
   }
   v = cmul(v, h);
   if (p.scat) {
@@ -538,11 +368,6 @@ __device__ __forceinline__ float2 prop_point(const ColParams& p, float2 v, int x
     G = fmaf(__ldg(p.gw + k), a2, G);
   }
   return cscale(v, p.scale);
-}
-
-// n*n*k0*k0 in the FP32 order of the kernels (bpm_3d_kernels.cl:425), no contraction
-__device__ __forceinline__ float prop_nk(const ColParams& p, float n_eff) {
-  return __fmul_rn(__fmul_rn(__fmul_rn(n_eff, n_eff), p.k0f), p.k0f);
 }
 
 template <int T>
@@ -929,38 +754,6 @@ __global__ void grad_parts_sum_kernel(float* grad, const float* part, long long 
   grad[i] = sacc;
 }
 
-// Weighted-mode sums (sum |u| dn, sum |u|). Every kernel of the sequence-in-registers family
-// adds them in one order, so all give the same bits: a lane over its rows t, t + 32, ..., the
-// lanes of a column by this tree, and the columns by weighted_total.
-__device__ __forceinline__ float2 lane_tree2(float2 a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
-    a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
-  }
-  return a;
-}
-
-// dn0 = sum |u| dn / sum |u| (mult_dn_mean_buff, bpm_3d_kernels.cl:117) from the column sums
-// get(c), c < nx: lane t adds columns t, t + 32, ... (fetched U at a time), then the tree;
-// called by whole warps
-template <int U, class Get>
-__device__ __forceinline__ float weighted_total(int nx, int t, Get get) {
-  float2 a = make_float2(0.f, 0.f);
-  for (int c = t; c < nx; c += 32 * U) {
-    float2 v[U];
-#pragma unroll
-    for (int k = 0; k < U; k++) v[k] = c + 32 * k < nx ? get(c + 32 * k) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      a.x += v[k].x;
-      a.y += v[k].y;
-    }
-  }
-  a = lane_tree2(a);
-  return a.x / a.y;
-}
-
 // the 16 column sums of a block of 512 threads in the coalesced tile mapping (r0, cc), from
 // the threads' sums over their rows: warp w ends up with column w's (all lanes). red: 16 x 33
 // float2 of shared memory that every thread is done reading.
@@ -997,58 +790,6 @@ struct ColSplitCfg {
   static constexpr size_t SMEM_DN = SMEM + (size_t)16 * N * sizeof(float);  // + dn slice 0 of the tile
   static constexpr size_t SMEM_KY = SMEM + (size_t)N * sizeof(float);       // + the ky^2 column
 };
-
-// the propagator on the thread's rows r0 + L i of column x (prop_point's arithmetic): the
-// row-major table H (conj(H) for the adjoint; TABLE) or the FP32 recipe with kx^2 of the
-// column and the ky^2 table staged in shared memory; with scattering sums
-// (bpm_3d.py:335-341) the thread's partials S, G over its rows
-template <int N, bool TABLE, bool SCAT, int L>
-__device__ __forceinline__ void propagate_rows_t(const ColParams& p, float2 (&v)[N / L], int x, int r0,
-                                                 float n_eff, float kx2, const float* sky2, float& S, float& G) {
-  const unsigned step = (unsigned)L * (unsigned)p.nx;
-  const unsigned off = (unsigned)r0 * (unsigned)p.nx + (unsigned)x;
-  const bool cj = p.conj_h;
-  const float nkx = TABLE ? 0.f : __fsub_rn(prop_nk(p, n_eff), kx2);
-  auto hval = [&](int i) {
-    float2 h;
-    if constexpr (TABLE) {
-      h = __ldg(p.H + off + i * step);
-      if (cj) h.y = -h.y;
-    } else {
-      const float tmp = __fsub_rn(nkx, sky2[r0 + L * i]);
-      h = make_float2(0.f, 0.f);
-      if (tmp >= 0.f) {
-        const float ph = __fmul_rn(-p.dzf, __fsqrt_rn(tmp));
-        sincosf(ph, &h.y, &h.x);
-      }
-    }
-    return h;
-  };
-  if constexpr (!SCAT) {
-#pragma unroll
-    for (int i = 0; i < N / L; i++) v[i] = cscale(cmul(v[i], hval(i)), p.scale);
-    return;
-  }
-  const float2 plain = (x == 0 && r0 == 0) ? plain_wave(p) : make_float2(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < N / L; i++) {
-    const float2 u = cmul(v[i], hval(i));
-    float2 d = u;
-    if (x == 0 && r0 == 0 && i == 0) d = csub(d, plain);
-    const float a2 = cabs2(d);
-    S = fmaf(__ldg(p.sw + off + i * step), a2, S);
-    G = fmaf(__ldg(p.gw + off + i * step), a2, G);
-    v[i] = cscale(u, p.scale);
-  }
-}
-template <int N, bool SCAT, int L>
-__device__ __forceinline__ void propagate_rows(const ColParams& p, float2 (&v)[N / L], int x, int r0,
-                                               float n_eff, float kx2, const float* sky2, float& S, float& G) {
-  if (p.prop_mode == 0)
-    propagate_rows_t<N, true, SCAT, L>(p, v, x, r0, n_eff, kx2, sky2, S, G);
-  else
-    propagate_rows_t<N, false, SCAT, L>(p, v, x, r0, n_eff, kx2, sky2, S, G);
-}
 
 // blocks per SM a column kernel of C columns x L threads must fit (registers as row_min_blocks)
 __host__ __device__ constexpr int col_min_blocks(int N, int L, int C) {
@@ -1372,7 +1113,6 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
 // rounding). Every wait is bounded in time; a block that gives up finishes the march without
 // further waits (its output is then wrong) and records it for bpm_device_status.
 // ---------------------------------------------------------------------------------------
-constexpr unsigned long long kClusterWaitNs = 2000000000ull;  // a wait gives up after 2 s
 __device__ int g_march_status;                                // nonzero once a wait gave up
 
 struct ClusterArgs {
@@ -1576,8 +1316,7 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
       float2 h = hc[m];
       if (!table) {
         const float tmp = __fsub_rn(nkx, hc[m].x);
-        h = make_float2(0.f, 0.f);
-        if (tmp >= 0.f) sincosf(__fmul_rn(-q.dzf, __fsqrt_rn(tmp)), &h.y, &h.x);
+        h = tmp >= 0.f ? cos_sin(__fmul_rn(-q.dzf, __fsqrt_rn(tmp))) : make_float2(0.f, 0.f);
       }
       v[m] = cscale(cmul(v[m], h), q.scale);
     }
@@ -1989,7 +1728,7 @@ int default_group(const bpm_plan* pl, int batch) {
 }
 
 struct WsLayout {
-  size_t w, red, dn0, scat, total;
+  size_t w, red, dn0, scat, counter, total;
 };
 
 WsLayout ws_layout(const bpm_plan* pl, int G) {
@@ -2003,7 +1742,9 @@ WsLayout ws_layout(const bpm_plan* pl, int G) {
   L.dn0 = off;
   off += align256((size_t)G * sizeof(float));
   L.scat = off;
-  off += align256((size_t)G * ntiles * 2 * sizeof(float));
+  off += align256((size_t)G * std::max(ntiles, kGridBlocks) * 2 * sizeof(float));
+  L.counter = off;
+  off += align256((size_t)G * kGridCounterStride * sizeof(unsigned));
   L.total = off;
   return L;
 }
@@ -2326,7 +2067,7 @@ struct ClusterK {
     a.cp = c.cp;
     a.u0 = static_cast<const float2*>(r->u0);
     a.nz = pl->d.nz;
-    a.wait_ns = kClusterWaitNs;
+    a.wait_ns = kMarchWaitNs;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = config((unsigned)r->batch, s, at);
     BPM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_march_kernel<N>, a));
@@ -2349,6 +2090,53 @@ int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaSt
   return kNotCluster;
 }
 
+// The whole march as one cooperative launch (march_grid.cu), for one or a few fields. Where it is
+// the default (GB300, us per step, against the pass kernels replayed as a graph):
+//   the weighted mode, up to 4 fields: 1024^2 22.7 against 31.2 for one field, 512^2 11.6 against
+//     16.1 (2 fields 13.1 against 17.5), 256 x 512 9.9 against 14.4, 256^2 7.6 against 9.6; 3 and 4
+//     fields of 256^2 stay with the cluster kernel (8.9 against 9.7 here);
+//   the other modes, up to 2 fields: 1024^2 17.9 against 20.9, 128 x 1024 11.3 against 12.9, 256 x
+//     512 6.6 against 7.2; 512^2 8.7 against 8.4 and 256^2 5.2 against 4.8 for one field, where
+//     the passes launched one by one take 8.6 and 5.7, so a march of one such field that is being
+//     captured into a graph keeps the passes.
+// It holds its share of every SM until the march ends, so requests that march beside others ask
+// for the pass kernels (bpm_request.cluster = 2). BPM_GB300_GRID=1 takes it wherever it fits, =0
+// nowhere.
+bool grid_default(const bpm_grid_desc& d, int batch, cudaStream_t s) {
+  static const int force = [] {
+    const char* e = getenv("BPM_GB300_GRID");
+    return !e ? -1 : (strcmp(e, "0") == 0 ? 0 : 1);
+  }();
+  if (force >= 0) return force == 1;
+  if (d.mean_mode == BPM_MEAN_WEIGHTED) return batch <= (d.nx == 256 && d.ny == 256 ? 2 : 4);
+  if (batch > 2) return false;
+  if (batch == 1 && d.nx < 1024 && d.nx >= d.ny) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone) return false;
+  }
+  return true;
+}
+
+constexpr int kNotGrid = 1;
+int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
+  const bpm_grid_desc& d = pl->d;
+  if (d.nx < 128 || d.ny < 128 || r->ckpt || r->cluster == 2 || r->group || r->conc || r->col_block || r->col_fuse ||
+      !grid_default(d, r->batch, s) || ((d.nx == 1024 || d.ny == 1024) && !warp1024_enabled()))
+    return kNotGrid;
+  const int G = group_size(pl, r);
+  if (G < r->batch || r->batch > grid_march_capacity(d.nx, d.ny)) return kNotGrid;
+  MarchCtx c = make_ctx(pl, r, ws, 0, r->batch);
+  GridMarchArgs a;
+  a.rp = c.rp;
+  a.rp.do_mask = r->dn_dtype != BPM_DN_NONE;
+  a.cp = c.cp;
+  a.u0 = static_cast<const float2*>(r->u0);
+  a.nz = d.nz;
+  a.counter = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + ws_layout(pl, G).counter);
+  a.wait_ns = kMarchWaitNs;
+  return grid_march_launch(d.nx, d.ny, a, r->batch, s);
+}
+
 // All groups of a request. With room for several workspace slots, groups march
 // concurrently on the plan's auxiliary streams (forked from and joined back to s through
 // events, which also captures into a CUDA graph as parallel branches), so one group's
@@ -2360,7 +2148,14 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
                   const HostSink* sink = nullptr) {
   int rc = check_workspace(pl, r, ws, ws_bytes);
   if (rc) return rc;
-  const int nz = pl->d.nz;
+  const bpm_grid_desc& d = pl->d;
+  const int nz = d.nz;
+  // the cluster kernel where it is the faster of the two (128^2), else the cooperative launch
+  const bool grid_first = !(d.nx == 128 && d.ny == 128) && r->cluster != 1;
+  if (grid_first && !sink) {
+    const int grc = try_grid_march(pl, r, ws, s);
+    if (grc != kNotGrid) return grc;
+  }
   {
     const int crc = try_cluster_march(pl, r, ws, s);
     if (crc != kNotCluster) {
@@ -2372,6 +2167,10 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
       }
       return BPM_OK;
     }
+  }
+  if (!grid_first && !sink) {
+    const int grc = try_grid_march(pl, r, ws, s);
+    if (grc != kNotGrid) return grc;
   }
   const int G = group_size(pl, r);
   const int ngroups = (r->batch + G - 1) / G;
@@ -2609,7 +2408,10 @@ int bpmgb::march_status(int clear, int* v) {
     const int zero = 0;
     BPM_CUDA_TRY(cudaMemcpyToSymbol(g_march_status, &zero, sizeof(int)));
   }
-  return BPM_OK;
+  int g = 0;
+  const int rc = grid_march_status(clear, &g);
+  *v |= g;
+  return rc;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -356,13 +356,13 @@ class Server:
         req = N.Request(B, _ptr(u0), _ptr(dn), kind, dn_stride, None, None,
                         _ptr(out), ok, Nz * Ny * Nx, _ptr(last), None, None, 0, 0, None, 0, _ptr(mask))
         if Nx == Ny == 128 and self._inflight:
-            # 128^2 fields march fastest on the pass kernels when they have the GPU to
-            # themselves (the library's choice); beside other launches they take the
-            # whole-march cluster kernel, which holds 8 SMs per field for the march instead
-            # of interleaving full-GPU passes with theirs (the same bits either way; GB300:
-            # the serving trace's p50 2.70 -> 2.57 ms, 48 mixed requests submitted at once
-            # 17.5 -> 17.1 ms)
+            # the whole-march cluster kernel, a few SMs per field, beside other launches
+            # whatever the batch (the library's own choice up to 32 fields)
             req.cluster = 1
+        elif min(Nx, Ny) >= 128:
+            # pass kernels, which interleave with the other streams' launches; the library's
+            # one-launch march would hold its part of every SM until the march ends
+            req.cluster = 2
         N.check(N.lib().bpm_propagate(plan.handle, ctypes.byref(req), _ptr(ws), wsb,
                                       ctypes.c_void_p(stream.cuda_stream)), "bpm_propagate")
         la.keep += [u0, dn, ws, mask]

@@ -560,3 +560,39 @@ def test_cluster_rule_does_not_change_a_result(bpm, side, mode, kind, batch):
         o = bpm_ref.bpm_3d((side, side, nz), (.1, .1, .1), u0=u0[b], precision="fp64", **kw)
         assert rel_l2(us, o) < TOL, b
     assert bpm._native.lib().bpm_device_status(0) == 0
+
+
+@pytest.mark.parametrize("size", [(128, 128, 5), (128, 1024, 4), (1024, 128, 4), (256, 128, 5), (256, 256, 2),
+                                  (256, 512, 4), (512, 128, 1), (512, 256, 5), (512, 1024, 3), (1024, 1024, 3)])
+def test_one_launch_march_matches_pass_kernels(bpm, size):
+    """The march of one or two fields as one cooperative launch (or, at 128x128, one cluster)
+    against the pass kernels (launch shape cluster = 2): the same bits for every mean mode, dn
+    kind and output, shared and per-field dn; and its scattering sums against the FP64 oracle
+    to the parity tolerance."""
+    Nx, Ny, Nz = size
+    rng = np.random.default_rng(Nx + Ny)
+    real = (.03 * rng.standard_normal((Nz, Ny, Nx))).astype(np.float32)
+    cplx = (real - 1j * np.abs(.002 * rng.standard_normal(real.shape))).astype(np.complex64)
+    x = .1 * np.arange(Nx)
+    u0 = np.exp(2j * np.pi * rng.uniform(-.3, .3, (2, 1, 1)) * x[None, None, :]).repeat(Ny, 1).astype(np.complex64)
+    for mode, dn, half, nb in [("weighted", real, False, 1), ("weighted", real, True, 2), ("simple", real, False, 1),
+                               ("ignore", cplx, False, 2), ("weighted", None, False, 1),
+                               ("weighted", np.stack([real, real[::-1]]), False, 2), ("ignore", real, False, 1)]:
+        for field, full in ((True, True), (False, True), (True, False)):
+            kw = dict(lam=.5, n0=1.33, u0=u0[:nb], dn=dn, mean_mode=mode, store_dn_as_half=half, absorbing_width=4,
+                      return_field=field, return_full=full)
+            n0 = bpm.launch_count()
+            one = bpm.bpm_3d_batched(size, (.1, .1, .1), **kw)
+            # a new plan, the phase masks, the march (two fields of the wider grids do not fit at once)
+            assert nb > 1 or bpm.launch_count() - n0 <= 3, (mode, nb)
+            assert np.array_equal(one, bpm.bpm_3d_batched(size, (.1, .1, .1), launch={"cluster": 2}, **kw)), (mode, nb)
+    assert bpm._native.lib().bpm_device_status(0) == 0
+    if Nz < 2 or Nx * Ny > 512 * 512:
+        return
+    for mode in ("weighted", "ignore"):
+        kw = dict(lam=.5, n0=1.33, u0=u0[1], dn=real, mean_mode=mode, return_scattering=True, return_g=True)
+        got = bpm.bpm_3d(size, (.1, .1, .1), **kw)
+        want = bpm_ref.bpm_3d(size, (.1, .1, .1), precision="fp64", **kw)
+        assert got[1][0] == 0 and np.isnan(got[2][0])
+        for k, lo in ((0, 0), (1, 1), (2, 1)):
+            assert rel_l2(got[k][lo:], want[k][lo:]) < TOL, (mode, k)
