@@ -3,8 +3,8 @@
 `propagate_exit(dn, u0, ...)` marches a batch of fields (illumination angles) through one
 refractive-index volume and returns their exit planes; it is a torch.autograd.Function
 whose backward is bpm_backward in libbpm_gb300.so: the forward march stores the field
-every `ckpt_every` planes, the backward recomputes each segment from its checkpoint and
-marches the adjoint field back with the conjugate propagator and conjugate phase masks,
+every `ckpt_every` planes (every plane where they take at most KEEP_ALL_BYTES), the
+backward recomputes each segment from its checkpoint (nothing then) and marches the adjoint field back with the conjugate propagator and conjugate phase masks,
 writing k0 dz Im(conj(G) u) per plane. The propagator must not depend on dn, so this is
 the "ignore" mean mode (the Bpm3d class semantics with prop="class", or bpm_3d's
 mean_mode="ignore" with prop="functional"). The reference has no gradient
@@ -19,6 +19,11 @@ from .bpm3d import _apply_launch, _ptr, _stream_ptr, get_plan, mask_pays, precom
 
 __all__ = ["propagate_exit"]
 
+# A forward march whose planes take no more than this keeps them all instead of one in
+# ckpt_every, and its backward pass recomputes nothing: a third of the marching. GB300, 16
+# fields of 256x256x128 (1.07 GB): @@ ms forward and backward.
+KEEP_ALL_BYTES = 2 << 30
+
 
 class _ExitMarch(torch.autograd.Function):
 
@@ -29,8 +34,15 @@ class _ExitMarch(torch.autograd.Function):
         dev = u0.device
         u0c = u0.detach().to(torch.complex64).contiguous()
         dnc = dn.detach().to(torch.float32).contiguous() if dn is not None else None
-        n_ckpt = (Nz - 1) // ckpt_every + 1
-        ckpt = torch.empty((B, n_ckpt, Ny, Nx), dtype=torch.complex64, device=dev)
+        ckpt = None
+        if B * Nz * Ny * Nx * 8 <= KEEP_ALL_BYTES:
+            try:
+                ckpt = torch.empty((B, Nz, Ny, Nx), dtype=torch.complex64, device=dev)
+                ckpt_every = 1
+            except torch.cuda.OutOfMemoryError:
+                pass
+        if ckpt is None:
+            ckpt = torch.empty((B, (Nz - 1) // ckpt_every + 1, Ny, Nx), dtype=torch.complex64, device=dev)
         last = torch.empty((B, Ny, Nx), dtype=torch.complex64, device=dev)
         kind = N.DN_F32 if dnc is not None else N.DN_NONE
         bstride = Nz * Ny * Nx if (dnc is not None and dnc.dim() == 4) else 0

@@ -2242,11 +2242,11 @@ BwLayout bw_layout(const bpm_plan* pl, int G, int k) {
   const size_t plane = (size_t)pl->d.nx * pl->d.ny;
   size_t off = 0;
   L.fwd = off;
-  off += ws_layout(pl, G).total;
+  if (k > 1) off += ws_layout(pl, G).total;
   L.adj = off;
   off += ws_layout(pl, G).total;
-  L.seg = off;
-  off += align256((size_t)G * (k + 1) * plane * sizeof(float2));
+  L.seg = off;  // with every plane kept (k = 1) the checkpoints are the forward fields
+  if (k > 1) off += align256((size_t)G * (k + 1) * plane * sizeof(float2));
   L.part = off;
   off += align256((size_t)bw_grad_parts(G) * pl->d.nz * plane * sizeof(float));
   L.total = off;
@@ -2333,8 +2333,13 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
     ca.cp.conj_h = 1;
     const float2* ck = static_cast<const float2*>(r->ckpt) + (size_t)b0 * n_ckpt * plane;
     const float2* gl = static_cast<const float2*>(grad_last) + (size_t)b0 * plane;
+    if (k == 1) {
+      ca.rp.seg = ck;
+      ca.rp.seg_bstride = (long long)n_ckpt * plane;
+    }
     for (int sgi = nseg - 1; sgi >= 0; sgi--) {
-      const int zs = sgi * k, ze = std::min(zs + k, nz - 1);
+      const int zs = k == 1 ? 0 : sgi * k, ze = k == 1 ? sgi + 1 : std::min(zs + k, nz - 1);
+      const int zstop = k == 1 ? sgi : zs;
       // recompute planes zs..ze of the forward march from checkpoint sgi
       RowParams rp = cf.rp;
       rp.src = ck + (size_t)sgi * plane;
@@ -2344,8 +2349,8 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
       rp.do_inv = 0;
       rp.do_fwd = 1;
       rp.do_mask = 0;
-      if ((rc = launch_row(d.nx, cf.grow, s, rp))) return rc;
-      for (int i = zs; i < ze; i++) {
+      if (k > 1 && (rc = launch_row(d.nx, cf.grow, s, rp))) return rc;
+      for (int i = zs; k > 1 && i < ze; i++) {
         cf.cp.z = i;
         if ((rc = launch_col<0>(d.ny, cf.gcol, s, cf.cp))) return rc;
         rp = cf.rp;
@@ -2356,8 +2361,8 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
         rp.do_mask = r->dn_dtype != BPM_DN_NONE;
         if ((rc = launch_row(d.nx, cf.grow, s, rp))) return rc;
       }
-      // march the adjoint from plane ze down to plane zs
-      for (int z = ze; z > zs; z--) {
+      // march the adjoint from plane ze down to plane zs (k = 1: one plane)
+      for (int z = ze; z > zstop; z--) {
         RowParams ra = ca.rp;
         ra.z = z;
         ra.seg_z0 = zs;

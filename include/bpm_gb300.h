@@ -257,8 +257,9 @@ size_t bpm_backward_workspace_bytes(const bpm_plan* plan, int batch, int group, 
  * grad_dn (nz, ny, nx) -- and, if grad_u0 is not NULL, the gradient
  * with respect to u0 into grad_u0 (batch, ny, nx) complex64. The request must be the one
  * the forward bpm_propagate ran with, including its checkpoints (req->ckpt,
- * req->ckpt_every): each segment between checkpoints is recomputed forward, then marched
- * backward with the conjugate propagator and conjugate phase masks.
+ * req->ckpt_every): each segment between checkpoints is recomputed forward (with
+ * ckpt_every = 1 the checkpoints are the fields and nothing is), then marched backward with
+ * the conjugate propagator and conjugate phase masks.
  * No reference counterpart (the reference has no gradient; bpm/bpm/bpm_3d_inverse.py is a
  * non-functional sketch). */
 int bpm_backward(bpm_plan* plan, const bpm_request* req, const void* grad_last, float* grad_dn,

@@ -181,3 +181,27 @@ def test_summed_gradient_matches_per_field_sum(torch_bpm, group):
     per_field = grad_of(dn0.expand(B, Nz, Ny, Nx).contiguous()).double().sum(dim=0)
     assert torch.all(g1[0] == 0)
     assert rel_l2(g1.double().cpu().numpy(), per_field.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("fields,nx,ny,nz,ckpt,shared", [(3, 128, 128, 9, 4, True), (9, 128, 64, 6, 5, True),
+                                                         (2, 64, 128, 5, 2, False), (1, 256, 128, 2, 16, True),
+                                                         (2, 128, 128, 1, 4, True)])
+def test_kept_planes_equal_recomputed_ones(monkeypatch, fields, nx, ny, nz, ckpt, shared):
+    """A march that keeps every plane and one that recomputes its segments from checkpoints give
+    the same exit planes and gradients, bit for bit."""
+    import torch
+    from bpm_gb300 import adjoint
+    g = torch.Generator(device="cuda").manual_seed(fields)
+    shape = (nz, ny, nx) if shared else (fields, nz, ny, nx)
+    dn0 = torch.rand(shape, device="cuda", generator=g) * .04
+    u0 = torch.exp(2j * np.pi * torch.rand((fields, 1, nx), device="cuda", generator=g)).expand(fields, ny, nx)
+    u0 = u0.to(torch.complex64).contiguous()
+    got = []
+    for keep in (1 << 40, 0):
+        monkeypatch.setattr(adjoint, "KEEP_ALL_BYTES", keep)
+        dn, u = dn0.clone().requires_grad_(True), u0.clone().requires_grad_(True)
+        out = adjoint.propagate_exit(dn, u, (nx, ny, nz), (.1, .1, .1), .5, 1.33, absorbing_width=3, ckpt_every=ckpt)
+        (out.abs() ** 4).sum().backward()
+        got.append((out.detach(), dn.grad, u.grad))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
