@@ -21,7 +21,7 @@ __all__ = ["propagate_exit"]
 
 # A forward march whose planes take no more than this keeps them all instead of one in
 # ckpt_every, and its backward pass recomputes nothing: a third of the marching. GB300, 16
-# fields of 256x256x128 (1.07 GB): @@ ms forward and backward.
+# fields of 256x256x128 (1.07 GB): 5.32 -> 3.62 ms forward and backward.
 KEEP_ALL_BYTES = 2 << 30
 
 

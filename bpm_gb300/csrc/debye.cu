@@ -570,6 +570,7 @@ __global__ void debye_assemble_kernel(int nx, int ny, int nz, OctGeom g, int M, 
   const int y = blockIdx.y, z = blockIdx.z;
   const int x = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (x >= nx) return;
+  dep_wait();
   const Voxel a = assemble_point<MIR>(x, y, z, nx, ny, nz, g, M, Zo, ex0, ey0, I, trig);
   const Voxel b = assemble_point<MIR>(x + 1, y, z, nx, ny, nz, g, M, Zo, ex0, ey0, I, trig);
   const size_t v = ((size_t)z * ny + y) * nx + x;  // even: 8-byte u pairs, 16-byte field pairs
@@ -616,6 +617,7 @@ __global__ void debye_scatter_kernel(int nx, int ny, int nz, OctGeom g, int M, i
   const int nyp = mirror_positions<MIR>(jy, ny, g.nyo, py);
   const int nzp = mirror_positions<MIR>(kz, nz, g.nzo, pz);
   if (nxp == 0 || nyp == 0 || nzp == 0) return;
+  dep_wait();
   const Voxel v = octant_sample(ix, jy, kz, g.nxo, M, Zo, ex0, ey0, I, trig);
 #pragma unroll
   for (int c = 0; c < 2; c++) {
@@ -660,19 +662,15 @@ int launch_assemble(const debye_desc* d, bool gauss, const OctGeom& g, int M, in
                     ((uintptr_t)ey & 15) == 0 && ((uintptr_t)ez & 15) == 0;
   if (fields && pair) {
     const dim3 grid((d->nx / 2 + 127) / 128, d->ny, d->nz);
-    if (gauss)
-      debye_assemble_kernel<MIR_GAUSS><<<grid, 128, 0, s>>>(d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex,
-                                                            pey, pez);
-    else
-      debye_assemble_kernel<MIR_STD><<<grid, 128, 0, s>>>(d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex,
-                                                          pey, pez);
+    BPM_CUDA_TRY(launch_dep(gauss ? debye_assemble_kernel<MIR_GAUSS> : debye_assemble_kernel<MIR_STD>, grid, dim3(128),
+                            0, s, d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex, pey, pez));
     BPM_LAUNCH_CHECK("debye_assemble_kernel");
     return BPM_OK;
   }
   const dim3 grid((g.nxo + 127) / 128, g.nyo, g.nzo);
   auto fn = gauss ? (fields ? debye_scatter_kernel<MIR_GAUSS, true> : debye_scatter_kernel<MIR_GAUSS, false>)
                   : (fields ? debye_scatter_kernel<MIR_STD, true> : debye_scatter_kernel<MIR_STD, false>);
-  fn<<<grid, 128, 0, s>>>(d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex, pey, pez);
+  BPM_CUDA_TRY(launch_dep(fn, grid, dim3(128), 0, s, d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex, pey, pez));
   BPM_LAUNCH_CHECK("debye_scatter_kernel");
   return BPM_OK;
 }
@@ -870,6 +868,7 @@ __device__ __forceinline__ int radius_column(int r, int nxo, bool sym) {
 // k r as a float pair). 32-thread blocks spread the FP64 chains over the SMs.
 __global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, int M, int nbn, double* ct,
                                       float* wf, float2* si2, float2* kr2, float* trig) {
+  dep_release();
   if ((int)blockIdx.x < nbn) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= T) return;
@@ -887,21 +886,24 @@ __global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, in
   }
 }
 
-// The operand tables of the product in one launch of 128-thread blocks: block (row, chunk)
-// takes nodes chunk*128 .. +127 of one row,
+// The operand tables of the product in one launch of 128-thread blocks: block (g, chunk) takes
+// nodes chunk*128 .. +127 of rpb rows from g*rpb on,
 //   rows [0, Zo): Bh/Bl(2z + {0, 1}, t) = high/low parts of (cos, sin)(kz_z cos t), the phase
 //     formed and reduced modulo 2 pi in FP64, its sine and cosine in FP32;
 //   rows Zo + r: A(n Mr + r, t) = p_n(t) J_n(kr sin t) for n = 0, 1, 2 (debye_bessel_kernel's
 //     values, x = kr sin t rounded to FP32 from the pair product).
-__global__ void debye_tables_tc_kernel(int T, int Tp, int Mr, int nxo, int sym, int Zo, float z1, float z2, double k,
-                                       const double* __restrict__ ct, const float2* __restrict__ si2,
-                                       const float2* __restrict__ kr2, const float* __restrict__ wf,
-                                       float* __restrict__ A, float* __restrict__ Bh, float* __restrict__ Bl) {
-  const int row = blockIdx.x;
+// A Bessel evaluation is about 65 instructions, so with one row a block the device spent the
+// launch placing blocks (42 570 of them at 256^3): up to 8 rows a block share the node's values.
+__global__ void __launch_bounds__(128) debye_tables_tc_kernel(
+    int T, int Tp, int Mr, int nxo, int sym, int Zo, int rpb, float z1, float z2, double k,
+    const double* __restrict__ ct, const float2* __restrict__ si2, const float2* __restrict__ kr2,
+    const float* __restrict__ wf, float* __restrict__ A, float* __restrict__ Bh, float* __restrict__ Bl) {
   const int t = blockIdx.y * 128 + threadIdx.x;
+  const int row0 = blockIdx.x * rpb, row1 = min(row0 + rpb, Zo + Mr);
+  dep_wait();
+  dep_release();
   if (t >= T) return;
-  if (row < Zo) {
-    const int z = row;
+  for (int z = row0; z < min(row1, Zo); z++) {
     const double kz = k * (double)(Zo == 1 ? z1 : coord_f32(z, z1, z2, Zo));
     const double arg = kz * ct[t];
     const double q = rint(arg * kInvTwoPi);
@@ -912,17 +914,22 @@ __global__ void debye_tables_tc_kernel(int T, int Tp, int Mr, int nxo, int sym, 
     Bl[o] = c - tf32_hi(c);
     Bh[o + Tp] = tf32_hi(sn);
     Bl[o + Tp] = sn - tf32_hi(sn);
-    return;
   }
-  const int r = row - Zo;
-  const int m = radius_column(r, nxo, sym != 0);
-  const float x = mul_pair(kr2[m], si2[t]);
-  float j0, j1, j2;
-  bessel_j012(x, j0, j1, j2);
-  const size_t o = (size_t)r * Tp + t, RT = (size_t)Mr * Tp;
-  A[o] = wf[t] * j0;
-  A[RT + o] = wf[T + t] * j1;
-  A[2 * RT + o] = wf[2 * T + t] * j2;
+  if (row1 <= Zo) return;
+  const float2 sv = si2[t];
+  const float w0 = wf[t], w1 = wf[T + t], w2 = wf[2 * T + t];
+  const size_t RT = (size_t)Mr * Tp;
+#pragma unroll 2
+  for (int row = max(row0, Zo); row < row1; row++) {
+    const int r = row - Zo;
+    const float x = mul_pair(kr2[radius_column(r, nxo, sym != 0)], sv);
+    float j0, j1, j2;
+    bessel_j012(x, j0, j1, j2);
+    float* o = A + (size_t)r * Tp + t;
+    o[0] = w0 * j0;
+    o[RT] = w1 * j1;
+    o[2 * RT] = w2 * j2;
+  }
 }
 
 constexpr int TC_BM = 128, TC_BK = 32, TC_THREADS = 128;
@@ -1016,8 +1023,10 @@ debye_accum_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
   volatile int* abortv = &abort_flag;
   int issued = 0;  // slices whose loads were issued (warp 0 lane 0)
 
+  dep_release();
   if (warp == 0 && lane == 0) {
     // ---- loads ----
+    dep_wait();  // the operand tables
     for (int kt = 0; kt < KT && !*abortv; kt++) {
       const int st = kt % S;
       if (kt >= S && !tc::mbar_wait(&empty[st], (uint32_t)(kt / S - 1) & 1u, a.wait_ns)) {
@@ -1357,8 +1366,11 @@ int run_octant_tc(const debye_desc* d, bool gauss, double sig, float* u, void* e
   debye_setup_tc_kernel<<<(unsigned)(nbn + (L.M + 31) / 32), 32, 0, s>>>(na, g, k, L.T, L.M, nbn, ct, wf, si2, kr2,
                                                                           trig);
   BPM_LAUNCH_CHECK("debye_setup_tc_kernel");
-  debye_tables_tc_kernel<<<dim3((unsigned)(L.Zo + L.Mr), (unsigned)tb), 128, 0, s>>>(
-      L.T, L.Tp, L.Mr, L.nxo, L.sym ? 1 : 0, L.Zo, g.z1, g.z2, k, ct, si2, kr2, wf, A, Bh, Bl);
+  // rows per block: blocks for a few waves of 16 on each of 152 SMs
+  const int rpb = (int)std::min<long long>(8, std::max<long long>(1, (long long)(L.Zo + L.Mr) * tb / (152 * 64)));
+  BPM_CUDA_TRY(launch_dep(debye_tables_tc_kernel, dim3((unsigned)((L.Zo + L.Mr + rpb - 1) / rpb), (unsigned)tb),
+                          dim3(128), 0, s, L.T, L.Tp, L.Mr, L.nxo, L.sym ? 1 : 0, L.Zo, rpb, g.z1, g.z2, k,
+                          (const double*)ct, (const float2*)si2, (const float2*)kr2, (const float*)wf, A, Bh, Bl));
   BPM_LAUNCH_CHECK("debye_tables_tc_kernel");
   TcArgs ta;
   ta.T = L.T;
@@ -1385,7 +1397,7 @@ int run_octant_tc(const debye_desc* d, bool gauss, double sig, float* u, void* e
   if (smem > TC_SMEM_MAX) { set_error("quadrature tile does not fit shared memory"); return BPM_ERR_SHAPE; }
   BPM_CUDA_TRY(tc_prepare());
   const dim3 grid(L.ntn, (rows + TC_BM - 1) / TC_BM);
-  debye_accum_tc_kernel<<<grid, TC_THREADS, smem, s>>>(mA, mBh, mBl, ta);
+  BPM_CUDA_TRY(launch_dep(debye_accum_tc_kernel, grid, dim3(TC_THREADS), smem, s, mA, mBh, mBl, ta));
   BPM_LAUNCH_CHECK("debye_accum_tc_kernel");
   if (u || ex || ey || ez) return launch_assemble(d, gauss, g, L.M, L.Zo, I, trig, u, ex, ey, ez, s);
   return BPM_OK;
