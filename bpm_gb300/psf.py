@@ -25,14 +25,15 @@ def _desc(shape3, units3, lam, NA, n0, n_integration_steps, ex0=1., ey0=0., quad
     """debye_desc for the C ABI; returns (desc, keep-alive NA array)."""
     if quadrature not in QUADRATURES:
         raise ValueError("quadrature must be 'reference' or 'physical'")
-    if np.isscalar(NA):
-        NA = [0., NA]
-    NA = [float(a) for a in np.asarray(NA, np.float64).ravel()]
+    if isinstance(NA, (float, int)) or np.isscalar(NA):
+        NA = [0., float(NA)]
+    elif not (type(NA) in (list, tuple) and all(type(a) is float for a in NA)):
+        NA = [float(a) for a in np.asarray(NA, np.float64).ravel()]
     assert len(NA) % 2 == 0
     na = (ctypes.c_double * len(NA))(*NA)
     desc = N.DebyeDesc(int(shape3[0]), int(shape3[1]), int(shape3[2]), float(units3[0]), float(units3[1]),
-                       float(units3[2]), float(lam), float(n0), ctypes.cast(na, ctypes.POINTER(ctypes.c_double)),
-                       len(NA), int(n_integration_steps), float(ex0), float(ey0), QUADRATURES[quadrature])
+                       float(units3[2]), float(lam), float(n0), na, len(NA), int(n_integration_steps), float(ex0),
+                       float(ey0), QUADRATURES[quadrature])
     return desc, na
 
 
@@ -145,6 +146,8 @@ def focus_field_debye_at(x, y, z, lam, NA, n0=1., n_integration_steps=200, devic
 
     def flat(a):
         t = a if isinstance(a, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(np.asarray(a, np.float32)))
+        if t.dtype == torch.float32 and t.device == dev and t.is_contiguous():
+            return t
         return t.to(device=dev, dtype=torch.float32).reshape(-1).contiguous()
     shp = tuple(x.shape)
     assert shp == tuple(y.shape) == tuple(z.shape)
@@ -156,16 +159,14 @@ def focus_field_debye_at(x, y, z, lam, NA, n0=1., n_integration_steps=200, devic
                          lambda: L.debye_focus_field_at(ctypes.byref(desc), None, None, None, 0, None, None, None,
                                                         None, None, 0, None),
                          desc, "debye_focus_field_at")
-    u = torch.empty(n, dtype=torch.float32, device=dev)
-    ex = torch.empty(n, dtype=torch.complex64, device=dev)
+    u = torch.empty(shp, dtype=torch.float32, device=dev)
+    ex = torch.empty(shp, dtype=torch.complex64, device=dev)
     ey = torch.empty_like(ex)
     ez = torch.empty_like(ex)
     N.check(L.debye_focus_field_at(ctypes.byref(desc), _ptr(xs), _ptr(ys), _ptr(zs), n, _ptr(u), _ptr(ex), _ptr(ey),
                                    _ptr(ez), _ptr(ws), wsb, _stream_ptr()), "debye_focus_field_at")
-    res = tuple(a.reshape(shp) for a in (u, ex, ey, ez))
-    if device:
-        return res
-    return tuple(_d2h(a) for a in res)
+    res = (u, ex, ey, ez)
+    return res if device else tuple(_d2h(a) for a in res)
 
 
 def psf(shape, units, lam, NA, n0=1., n_integration_steps=200, return_field=False, device=False,
