@@ -77,6 +77,7 @@ SIGNATURES = {
     "bpm_workspace_bytes_conc": (c_size, [c_vp, c_int, c_int, c_int]),
     "bpm_propagate": (c_int, [c_vp, ctypes.POINTER(Request), c_vp, c_size, c_vp]),
     "bpm_mask_precompute": (c_int, [c_vp, c_vp, c_int, c_vp, c_vp]),
+    "bpm_slice_means": (c_int, [c_vp, c_int, c_int, c_int, c_double, c_vp, c_vp, c_vp]),
     "bpm_propagate_noalloc": (c_int, [c_vp, ctypes.POINTER(Request), c_vp]),
     "bpm_propagate_to_host": (c_int, [c_vp, ctypes.POINTER(Request), c_vp, c_int, c_vp, c_size, c_vp]),
     "bpm_launch_pass": (c_int, [c_vp, ctypes.POINTER(Request), c_vp, c_size, c_int, c_int, c_vp]),

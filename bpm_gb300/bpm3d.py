@@ -180,7 +180,14 @@ def _dn_kind(dn, store_dn_as_half):
 
 def _slice_tables(dn, n0, dev):
     """Per-slice float32(n0 + mean(dn[z])) and float32(mean(dn[z])) for mean_mode='simple'
-    (bpm_3d.py:216-220, :288-293): the slice means are taken on the caller's dn, in FP64."""
+    (bpm_3d.py:216-220, :288-293): the slice means are taken on the caller's dn, in FP64
+    (to FP64 accuracy on the device for a resident float32 volume, bpm_slice_means)."""
+    if _is_tensor(dn) and dn.dtype == torch.float32 and dn.device == dev and dn.is_contiguous() and dn.dim() == 3 \
+            and 0 < dn.numel() and dn.shape[0] <= 65535:
+        sn, sd = torch.empty((2, dn.shape[0]), dtype=torch.float32, device=dev)
+        N.check(N.lib().bpm_slice_means(_ptr(dn), int(dn.shape[2]), int(dn.shape[1]), int(dn.shape[0]), float(n0),
+                                        _ptr(sn), _ptr(sd), _stream_ptr()), "bpm_slice_means")
+        return sn, sd
     if dn is None:
         m = np.zeros(1, np.float64)
     elif _is_tensor(dn):

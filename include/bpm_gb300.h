@@ -235,6 +235,12 @@ int bpm_launch_pass(bpm_plan* plan, const bpm_request* req, void* workspace, siz
  * saves every field of a batch from re-evaluating them; (nz, ny, nx) complex64 output. */
 int bpm_mask_precompute(bpm_plan* plan, const void* dn, int dn_dtype, void* mask, void* stream);
 
+/* Slice tables of BPM_MEAN_SIMPLE from a device float32 volume (nz, ny, nx), nz <= 65535:
+ * slice_dn0[z] = float32(mean(dn[z])), slice_n[z] = float32(n0 + mean(dn[z])), the means to
+ * FP64 accuracy (bpm/bpm/bpm_3d.py:216-220, :288-293, where they are taken on the host). */
+int bpm_slice_means(const float* dn, int nx, int ny, int nz, double n0, float* slice_n, float* slice_dn0,
+                    void* stream);
+
 /* Capture the launches of bpm_propagate for a fixed request and workspace into a CUDA
  * graph; bpm_exec_launch replays it on any stream. The buffers named by `req` and the
  * workspace must stay valid and unchanged in address while the exec lives. No reference

@@ -596,3 +596,22 @@ def test_one_launch_march_matches_pass_kernels(bpm, size):
         assert got[1][0] == 0 and np.isnan(got[2][0])
         for k, lo in ((0, 0), (1, 1), (2, 1)):
             assert rel_l2(got[k][lo:], want[k][lo:]) < TOL, (mode, k)
+
+
+@pytest.mark.parametrize("shape,offset", [((1, 16, 16), 0), ((7, 128, 64), 0), ((3, 64, 32), 1), ((2, 1024, 1024), 0),
+                                          ((5, 3, 7), 2)])
+def test_slice_means_match_fp64(bpm, shape, offset):
+    """The device's slice tables against numpy's FP64 means, rounded once to float32: equal but
+    for a last bit where the sums' 2^-45 crosses a rounding boundary (volumes of every
+    alignment; values of both signs over six decades, with an offset that cancels)."""
+    import torch
+    from bpm_gb300.bpm3d import _slice_tables
+    rng = np.random.default_rng(shape[1])
+    a = (rng.standard_normal(shape) * 10. ** rng.uniform(-6, 0, shape) + .01).astype(np.float32)
+    buf = torch.zeros(a.size + offset, device="cuda")
+    dn = buf[offset:].reshape(shape)
+    dn.copy_(torch.from_numpy(a))
+    sn, sd = _slice_tables(dn, 1.33, buf.device)
+    m = a.astype(np.float64).mean(axis=(1, 2))
+    for got, want in ((sn, (1.33 + m).astype(np.float32)), (sd, m.astype(np.float32))):
+        assert np.all(np.abs(got.cpu().numpy().view(np.int32) - want.view(np.int32)) <= 1)
