@@ -672,7 +672,7 @@ row_shared_kernel(RowParams p, int nfields, int fw_rt) {
   const size_t zoff = (size_t)p.z * plane;
   for (int k = threadIdx.x; k < WarpFft<N, L>::TW; k += T) tw[k] = p.wtw[k];  // plan constant
   dep_wait();
-  dep_release();
+  if (p.early) dep_release();
   {
     const int es = PRE ? 8 : (p.dn_dtype == BPM_DN_C64 ? 8 : (p.dn_dtype == BPM_DN_F16 ? 2 : 4));
     const char* srcm = PRE ? reinterpret_cast<const char*>(p.mask + zoff + (size_t)y * N)
@@ -749,7 +749,7 @@ row_adj_shared_kernel(RowParams p, int nfields, int fw) {
   const size_t zoff = (size_t)p.z * plane;
   for (int k = threadIdx.x; k < WarpFft<N, L>::TW; k += T) tw[k] = p.wtw[k];  // plan constant
   dep_wait();
-  dep_release();
+  if (p.early) dep_release();
   {
     const int es = PRE ? 8 : (p.dn_dtype == BPM_DN_F16 ? 2 : 4);
     const char* srcm = PRE ? reinterpret_cast<const char*>(p.mask + zoff + (size_t)y * N)
@@ -900,7 +900,7 @@ col_split_kernel(ColParams p) {
   }
   float* sky2 = reinterpret_cast<float*>(smem + Cfg::DN_F2);
   dep_wait();
-  dep_release();
+  if (p.early) dep_release();
   // weighted reduction: dn slice 0 of this tile goes to shared memory with cp.async now and
   // is read after the transform; a 16-value row is 2^lg 16-byte pieces
   const char* dn_stage = nullptr;
@@ -1458,11 +1458,13 @@ int sm_count() {
   return n;
 }
 
-// Shared memory per SM that the passes of a march need with all the blocks resident that could
-// be, of `conc` groups at once: while t_need is set, pass_launch notes a pass's need instead of
-// launching it.
+// What the passes of a march need of an SM, with `conc` groups at once: while t_need is set,
+// pass_launch notes a pass's need instead of launching it.
 struct PassNeed {
-  size_t bytes, conc;
+  size_t conc;
+  int n;
+  double bytes[8];  // shared memory of the blocks that could be resident
+  double room[8];   // the share of the SM's registers and threads that they take
 };
 thread_local PassNeed* t_need = nullptr;
 
@@ -1475,11 +1477,17 @@ template <typename... KArgs, typename... Args>
 int pass_launch(const char* what, int carve, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                 cudaStream_t s, Args&&... args) {
   if (t_need) {
+    cudaFuncAttributes fa;
     int occ = 0;
+    BPM_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
     BPM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block.x, smem));
-    const size_t blocks = t_need->conc * grid.x * grid.y, per_sm = (blocks + sm_count() - 1) / sm_count();
-    // 1.5 KB a block for the system's share and static arrays
-    t_need->bytes = std::max(t_need->bytes, std::min<size_t>(occ, per_sm) * (smem + 1536));
+    const size_t blocks = t_need->conc * grid.x * grid.y;
+    const double n = (double)std::min<size_t>(occ, (blocks + sm_count() - 1) / sm_count());
+    const double room = std::max({(double)fa.numRegs * block.x / 65536, block.x / 2048., 1 / 32.});
+    if (t_need->n < 8) {
+      t_need->bytes[t_need->n] = n * (double)(smem + fa.sharedSizeBytes + 1024);  // 1 KB a block is the system's
+      t_need->room[t_need->n++] = n * room;
+    }
     return BPM_OK;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1499,16 +1507,40 @@ int pass_launch(const char* what, int carve, void (*kernel)(KArgs...), dim3 grid
   return BPM_OK;
 }
 
-// The partition for a march whose passes `passes` enqueues (each once) and of which `conc` groups
-// run at the same time
+// How the passes of a march are launched.
+// early: a pass lets the next one start as soon as its own inputs are there (else as its blocks
+// leave). The blocks that arrive early wait, and take the places that are free at
+// that moment: with one field, whose blocks leave most of every SM free, or with passes that fill
+// the device that is the shorter way; in between they gather on the SMs that happen to have room
+// and the pass after that takes up to twice as long (GB300, us per step, late against early: 4
+// fields of 512^2 without the sums 14.2 against 15.3, 14 of 64 x 512 10.0 against 17.8, 6 of 256 x
+// 512 12.5 against 17.4; one field of 512^2 9.6 against 8.2).
+// carve: the shared-memory partition that all passes ask for (see pass_launch): what the most
+// demanding pass needs, and with blocks arriving early what any two need side by side as far as
+// registers and threads let them be resident together. The largest partition, with the L1 cache at
+// its smallest, makes the 512^2 batches 3 % slower. A single field of 1024 columns, whose row
+// blocks hold twice the registers, takes the driver's choice (1024 x 256 9.9 against 12.7).
+struct PassPlan {
+  int carve, early;
+};
 template <class F>
-int march_carve(int conc, F passes) {
-  PassNeed need{0, (size_t)conc};
+PassPlan plan_passes(int nx, int fields, int conc, F passes) {
+  if (fields == 1 && nx == 1024) return {0, 1};
+  PassNeed need{(size_t)conc, 0, {}, {}};
   t_need = &need;
   const int rc = passes();
   t_need = nullptr;
-  constexpr size_t kMax = 228 * 1024;
-  return rc != BPM_OK ? 0 : std::max(1, (int)((100 * std::min(need.bytes, kMax) + kMax - 1) / kMax));
+  if (rc != BPM_OK) return {0, 1};
+  double most = 0., room = 0.;
+  for (int i = 0; i < need.n; i++) room = std::max(room, need.room[i]);
+  const int early = fields == 1 || room > .95;
+  for (int i = 0; i < need.n; i++)
+    for (int j = 0; j < need.n; j++) {
+      const double left = early ? std::max(0., 1. - need.room[i]) : 0.;
+      most = std::max(most, need.bytes[i] + (i == j ? 0. : need.bytes[j] * std::min(1., left / need.room[j])));
+    }
+  constexpr double kMax = 228 * 1024;
+  return {std::max(1, (int)std::ceil(100. * std::min(most, kMax) / kMax)), early};
 }
 
 template <int N>
@@ -1993,6 +2025,7 @@ MarchCtx make_ctx(const bpm_plan* pl, const bpm_request* r, void* ws, int b0, in
 
   cp.col_block = r->col_block;
   cp.col_fuse = r->col_fuse;
+  rp.early = cp.early = 1;
   c.grow = dim3(ny / 16, Gc);
   c.gcol = dim3(nx / 16, Gc);
   return c;
@@ -2183,14 +2216,17 @@ int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaSt
 }
 
 // The whole march as one cooperative launch (march_grid.cu), for one or a few fields. Where it is
-// the default (GB300, us per step, against the pass kernels replayed as a graph):
+// the default (GB300, us per step, against the pass kernels replayed as a graph; launched one by
+// one they take 0.2 to 0.3 us more a pass):
 //   the weighted mode, up to 4 fields: 1024^2 22.7 against 31.2 for one field, 512^2 11.6 against
-//     16.1 (2 fields 13.1 against 17.5), 256 x 512 9.9 against 14.4, 256^2 7.6 against 9.6; 3 and 4
-//     fields of 256^2 stay with the cluster kernel (8.9 against 9.7 here);
-//   the other modes, up to 2 fields: 1024^2 17.9 against 20.9, 128 x 1024 11.3 against 12.9, 256 x
-//     512 6.6 against 7.2; 512^2 8.7 against 8.4 and 256^2 5.2 against 4.8 for one field, where
-//     the passes launched one by one take 8.6 and 5.7, so a march of one such field that is being
-//     captured into a graph keeps the passes.
+//     15.6 (2 fields 13.1 against 17.4), 256 x 512 9.8 against 14.1, 256^2 7.6 against 9.5, 4 of
+//     512 x 256 12.2 against 12.9; 3 and 4 fields of 256^2 stay with the cluster kernel (8.9
+//     against 9.7 here);
+//   the other modes, one field of at least 256 columns: 1024^2 17.9 against 20.4, 512^2 8.7 against
+//     8.2, 512 x 256 6.6 against 6.2, 256^2 5.1 against 4.8, 128 x 1024 11.3 against 9.0; below 1024
+//     x 512 only where the passes would be launched one by one, and a march that is being captured
+//     into a graph keeps them; two fields from 512 columns on (512^2 9.8 against 11.0, 512 x 256
+//     7.3 against 7.7, 256^2 5.8 against 5.8).
 // It holds its share of every SM until the march ends, so requests that march beside others ask
 // for the pass kernels (bpm_request.cluster = 2). BPM_GB300_GRID=1 takes it wherever it fits, =0
 // nowhere.
@@ -2201,8 +2237,8 @@ bool grid_default(const bpm_grid_desc& d, int batch, cudaStream_t s) {
   }();
   if (force >= 0) return force == 1;
   if (d.mean_mode == BPM_MEAN_WEIGHTED) return batch <= (d.nx == 256 && d.ny == 256 ? 2 : 4);
-  if (batch > 2) return false;
-  if (batch == 1 && d.nx < 1024 && d.nx >= d.ny) {
+  if (batch > 2 || d.nx < (batch == 1 ? 256 : 512)) return false;
+  if (batch == 1 && !(d.nx == 1024 && d.ny >= 512)) {
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone) return false;
   }
@@ -2278,6 +2314,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   for (int w0 = 0; w0 < ngroups; w0 += conc) {
     const int nwave = std::min(conc, ngroups - w0);
     MarchCtx c[kMaxConcurrentGroups];
+    PassPlan pp{0, 1};
     int b0[kMaxConcurrentGroups], Gc[kMaxConcurrentGroups], zdone[kMaxConcurrentGroups];
     for (int j = 0; j < nwave; j++) {
       b0[j] = (w0 + j) * G;
@@ -2285,12 +2322,13 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
       zdone[j] = 0;
       c[j] = make_ctx(pl, r, static_cast<char*>(ws) + (size_t)j * slot, b0[j], Gc[j]);
       if (j == 0)
-        c[0].rp.carve = march_carve(nwave, [&] {
+        pp = plan_passes(d.nx, r->batch, nwave, [&] {
           int e = launch_first_row(pl, r, c[0], b0[0], st[0]);
           if (!e && nz > 1) e = launch_cols(pl, c[0], 0, 0, st[0]);
           return e || nz == 1 ? e : launch_row_z(pl, r, c[0], 1, st[0]);
         });
-      c[j].rp.carve = c[j].cp.carve = c[0].rp.carve;
+      c[j].rp.carve = c[j].cp.carve = pp.carve;
+      c[j].rp.early = c[j].cp.early = pp.early;
       if ((rc = launch_first_row(pl, r, c[j], b0[j], st[j]))) return rc;
     }
     for (int i = 0; i + 1 < nz || (i == 0 && nz == 1); i++) {
@@ -2436,7 +2474,7 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
       ca.rp.seg = ck;
       ca.rp.seg_bstride = (long long)n_ckpt * plane;
     }
-    cf.rp.carve = march_carve(1, [&] {
+    const PassPlan pp = plan_passes(d.nx, r->batch, 1, [&] {
       RowParams m = ca.rp;
       m.z = 1;
       m.do_inv = m.do_fwd = 1;
@@ -2449,7 +2487,8 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
       w.do_mask = m.do_mask;
       return e || k == 1 ? e : launch_row(d.nx, cf.grow, s, w);
     });
-    cf.cp.carve = ca.rp.carve = ca.cp.carve = cf.rp.carve;
+    cf.rp.carve = cf.cp.carve = ca.rp.carve = ca.cp.carve = pp.carve;
+    cf.rp.early = cf.cp.early = ca.rp.early = ca.cp.early = pp.early;
     for (int sgi = nseg - 1; sgi >= 0; sgi--) {
       const int zs = k == 1 ? 0 : sgi * k, ze = k == 1 ? sgi + 1 : std::min(zs + k, nz - 1);
       const int zstop = k == 1 ? sgi : zs;

@@ -79,6 +79,7 @@ struct RowParams {
   long long grad_part_stride;
   int grad_acc;
   int carve;                // host: shared-memory partition of the march's launches (percent, 0: the driver's choice)
+  int early;                // the next pass may start as soon as this one's inputs are there
 };
 
 __device__ __forceinline__ float load_dn_real(const void* dn, int dtype, size_t idx) {
@@ -160,7 +161,7 @@ struct ColParams {
   int dn_stage;              // weighted: dn rows may be staged with 16-byte cp.async
   int col_block;             // 0: the library's rule; 4, 8 or 16 columns per non-weighted block
   int col_fuse;              // weighted: 1 one fused column pass where available, 0 or 2 two passes
-  int carve;                 // host: as RowParams::carve
+  int carve, early;          // as in RowParams
 };
 
 template <int T>
