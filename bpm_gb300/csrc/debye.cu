@@ -231,15 +231,16 @@ __host__ __device__ constexpr double hankel_a(int n, int k) {
   return a;
 }
 
-// Taylor coefficients of J0 and J2 for 0 <= x < 16 in intervals of width 1/4: row i covers
+// Taylor coefficients of J0, J1 and J2 for 0 <= x < 16 in intervals of width 1/4: row i covers
 // [i/4, i/4 + 1/4) about its middle (row 0 about x = 0, so that J1 and J2 keep their relative
-// accuracy there), c[0..1][i] the eight coefficients of J0, c[2..3][i] those of J2, lowest
-// power first. Values at the middle come from the power series in FP64, the higher
-// coefficients from Bessel's equation x^2 y'' + x y' + (x^2 - n^2) y = 0 written about it.
+// accuracy there). c[2n][i] and c[2n + 1][i] are J_n's coefficients up to the sixth power, lowest
+// first, and what the float of the constant one leaves out. Values at the middle come from the
+// power series in FP64, the higher coefficients from Bessel's equation x^2 y'' + x y' + (x^2 -
+// n^2) y = 0 written about it.
 constexpr int BT_ROWS = 64;
 constexpr float BT_END = 16.f;
 struct BesselTaylor {
-  float4 c[4][BT_ROWS];
+  float4 c[6][BT_ROWS];
 };
 
 constexpr double bessel_series(int n, double x) {  // sum_k (-1)^k (x/2)^(2k+n) / (k! (k+n)!)
@@ -255,29 +256,27 @@ constexpr double bessel_series(int n, double x) {  // sum_k (-1)^k (x/2)^(2k+n) 
 
 constexpr BesselTaylor bessel_taylor() {
   BesselTaylor t{};
-  for (int i = 0; i < BT_ROWS; i++) {
-    double a[8] = {}, b[8] = {};
-    if (i == 0) {
-      a[0] = 1., a[2] = -1. / 4., a[4] = 1. / 64., a[6] = -1. / 2304.;
-      b[2] = 1. / 8., b[4] = -1. / 96., b[6] = 1. / 3072.;
-    } else {
-      const double c = .25 * i + .125;
-      const double j1 = bessel_series(1, c);
-      a[0] = bessel_series(0, c), a[1] = -j1;
-      b[0] = bessel_series(2, c), b[1] = j1 - 2. * b[0] / c;
-      for (int n = 0; n < 4; n += 2) {
-        double* y = n ? b : a;
-        for (int m = 0; m < 6; m++)
+  for (int n = 0; n < 3; n++)
+    for (int i = 0; i < BT_ROWS; i++) {
+      double y[7] = {};
+      if (i == 0) {
+        double term = n == 0 ? 1. : (n == 1 ? .5 : .125);  // 1 / (2^n n!)
+        for (int k = 0; 2 * k + n < 7; k++) {
+          y[2 * k + n] = term;
+          term /= -4. * (k + 1.) * (k + 1. + n);
+        }
+      } else {
+        const double c = .25 * i + .125;
+        y[0] = bessel_series(n, c);
+        y[1] = n == 0 ? -bessel_series(1, c) : bessel_series(n - 1, c) - n * y[0] / c;
+        for (int m = 0; m < 5; m++)
           y[m + 2] = -(c * (m + 1.) * (2. * m + 1.) * y[m + 1] + (m * m + c * c - n * n) * y[m] +
                        (m > 0 ? 2. * c * y[m - 1] : 0.) + (m > 1 ? y[m - 2] : 0.)) /
                      (c * c * (m + 2.) * (m + 1.));
       }
+      t.c[2 * n][i] = float4{(float)y[0], (float)y[1], (float)y[2], (float)y[3]};
+      t.c[2 * n + 1][i] = float4{(float)y[4], (float)y[5], (float)y[6], (float)(y[0] - (double)(float)y[0])};
     }
-    t.c[0][i] = float4{(float)a[0], (float)a[1], (float)a[2], (float)a[3]};
-    t.c[1][i] = float4{(float)a[4], (float)a[5], (float)a[6], (float)a[7]};
-    t.c[2][i] = float4{(float)b[0], (float)b[1], (float)b[2], (float)b[3]};
-    t.c[3][i] = float4{(float)b[4], (float)b[5], (float)b[6], (float)b[7]};
-  }
   return t;
 }
 __device__ const BesselTaylor g_bessel = bessel_taylor();
@@ -289,26 +288,20 @@ __device__ const BesselTaylor g_bessel = bessel_taylor();
 // sin chi_1 = -cos chi_0; 1/x and the envelope come from the approximate reciprocal and
 // reciprocal square root (2 ulp, far below what the truncated series resolves), and J2 from
 // the recurrence 2 J1/x - J0 with that reciprocal. Below 16 the Taylor polynomials of
-// g_bessel, J1 as minus the derivative of J0's: no branch and no division, absolute errors
-// below 1e-7 against FP64 over [0, 16).
+// g_bessel: no branch and no division, absolute errors below 5e-8 against FP64 over [0, 16).
 __device__ __forceinline__ void bessel_j012(float x, float& j0, float& j1, float& j2) {
   const float ax = fabsf(x);
   if (ax < BT_END) {
     const int i = (int)(ax * 4.f);
-    const float4 a = __ldg(&g_bessel.c[0][i]), b = __ldg(&g_bessel.c[1][i]);
-    const float4 e = __ldg(&g_bessel.c[2][i]), f = __ldg(&g_bessel.c[3][i]);
     const float d = ax - (i > 0 ? fmaf(.25f, (float)i, .125f) : 0.f);
-    // value p and derivative q of J0's polynomial in one pass
-    float p = b.w, q = b.w;
-    p = fmaf(p, d, b.z), q = fmaf(q, d, p);
-    p = fmaf(p, d, b.y), q = fmaf(q, d, p);
-    p = fmaf(p, d, b.x), q = fmaf(q, d, p);
-    p = fmaf(p, d, a.w), q = fmaf(q, d, p);
-    p = fmaf(p, d, a.z), q = fmaf(q, d, p);
-    p = fmaf(p, d, a.y), q = fmaf(q, d, p);
-    j0 = fmaf(p, d, a.x);
-    j1 = x < 0.f ? q : -q;
-    j2 = fmaf(fmaf(fmaf(fmaf(fmaf(fmaf(fmaf(f.w, d, f.z), d, f.y), d, f.x), d, e.w), d, e.z), d, e.y), d, e.x);
+    auto poly = [&](int n) {
+      const float4 a = __ldg(&g_bessel.c[2 * n][i]), b = __ldg(&g_bessel.c[2 * n + 1][i]);
+      return a.x + fmaf(fmaf(fmaf(fmaf(fmaf(fmaf(b.z, d, b.y), d, b.x), d, a.w), d, a.z), d, a.y), d, b.w);
+    };
+    j0 = poly(0);
+    const float j1a = poly(1);
+    j1 = x < 0.f ? -j1a : j1a;
+    j2 = poly(2);
     return;
   }
   const float r = __fdividef(1.f, ax), y = r * r;
