@@ -105,20 +105,36 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
     }
     __syncthreads();
   };
-  // the warp's mask row of plane z into shared memory, each lane the elements it will use:
-  // asynchronous copies of precomputed masks, else formed from dn now
+  // the warp's row of plane z's masks (or of dn) into shared memory, each lane the elements it
+  // will use, asynchronously (half values by ordinary loads)
   auto stage_mask = [&](int z) {
     if (!in_row || !p.do_mask || z >= nz) return;
     const size_t off = (size_t)z * plane + (size_t)y * NX + t;
-#pragma unroll 4
-    for (int m = 0; m < EX; m++) {
-      if (p.mask)
-        cp_async8(mrow + t + 32 * m, p.mask + off + 32 * m);
-      else
-        mrow[t + 32 * m] = mask_value(p.dn, p.dn_dtype, gl * p.dn_bstride + off + 32 * m, p.unit_k, t + 32 * m, y, NX,
-                                      NY, p.absorb, p.taper);
+    if (p.mask || p.dn_dtype == BPM_DN_C64) {
+      const float2* src = p.mask ? p.mask + off : reinterpret_cast<const float2*>(p.dn) + gl * p.dn_bstride + off;
+#pragma unroll
+      for (int m = 0; m < EX; m++) cp_async8(mrow + t + 32 * m, src + 32 * m);
+    } else if (p.dn_dtype == BPM_DN_F32) {
+      const float* src = reinterpret_cast<const float*>(p.dn) + gl * p.dn_bstride + off;
+#pragma unroll
+      for (int m = 0; m < EX; m++) cp_async4(mrow + t + 32 * m, src + 32 * m);
+    } else {
+      const __half* src = reinterpret_cast<const __half*>(p.dn) + gl * p.dn_bstride + off;
+#pragma unroll
+      for (int m = 0; m < EX; m++) mrow[t + 32 * m].x = __half2float(src[32 * m]);
     }
     cp_async_commit();
+  };
+  // the masks of the staged dn row in its place
+  auto form_mask = [&] {
+    if (!in_row || !p.do_mask || p.mask) return;
+    cp_async_wait<0>();
+#pragma unroll 4
+    for (int m = 0; m < EX; m++) {
+      float2& e = mrow[t + 32 * m];
+      e = p.dn_dtype == BPM_DN_C64 ? mask_from_complex(e, p.unit_k)
+                                   : mask_from_real(e.x, p.unit_k, t + 32 * m, y, NX, NY, p.absorb, p.taper);
+    }
   };
   auto store_plane = [&](int z, const float2 (&u)[EX]) {
     const size_t pix = (size_t)y * NX + t, o = (size_t)z * plane + pix;
@@ -313,6 +329,7 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
       o[1] = G;
     }
     arrive();
+    form_mask();
   }
   cp_async_wait<0>();
 }

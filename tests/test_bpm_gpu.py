@@ -615,3 +615,38 @@ def test_slice_means_match_fp64(bpm, shape, offset):
     m = a.astype(np.float64).mean(axis=(1, 2))
     for got, want in ((sn, (1.33 + m).astype(np.float32)), (sd, m.astype(np.float32))):
         assert np.all(np.abs(got.cpu().numpy().view(np.int32) - want.view(np.int32)) <= 1)
+
+
+@pytest.mark.parametrize("kind", ["f32", "f16", "c64"])
+@pytest.mark.parametrize("size,absorb", [((16, 16, 1), 0), ((128, 32, 3), 5), ((1024, 512, 3), 7)])
+def test_mask_precompute_aligned_and_unaligned(bpm, kind, size, absorb):
+    """The precomputed masks from 16-byte aligned buffers (four voxels a thread) and from buffers
+    8 bytes off (one) are the same bits, and the FP64 formula to 3e-7: the phase k0 dz dn (below
+    0.2) rounded to FP32 twice, sine and cosine within 1.6 ulp, the taper's product."""
+    import ctypes
+    import torch
+    from bpm_gb300 import _native as N
+    from bpm_gb300.bpm3d import get_plan
+    nx, ny, nz = size
+    rng = np.random.default_rng(nx)
+    a = rng.uniform(-.1, .1, (nz, ny, nx))
+    dt = {"f32": torch.float32, "f16": torch.float16, "c64": torch.complex64}[kind]
+    a = torch.from_numpy(a - 1j * rng.uniform(0, .01, a.shape) if kind == "c64" else a).to(dt)
+    plan = get_plan(size, (.1, .1, .1), .5, 1.33, absorb, "ignore")
+    got = []
+    for off in (0, 8):
+        buf = torch.zeros(a.numel() * a.element_size() + 16, dtype=torch.uint8, device="cuda")
+        out = torch.zeros(a.numel() * 8 + 16, dtype=torch.uint8, device="cuda")
+        dn = buf[off:off + a.numel() * a.element_size()].view(dt)
+        dn.copy_(a.reshape(-1))
+        N.check(N.lib().bpm_mask_precompute(plan.handle, ctypes.c_void_p(dn.data_ptr()),
+                                            {"f32": N.DN_F32, "f16": N.DN_F16, "c64": N.DN_C64}[kind],
+                                            ctypes.c_void_p(out.data_ptr() + off), None))
+        torch.cuda.synchronize()
+        got.append(out[off:off + a.numel() * 8].view(torch.complex64).cpu().numpy().reshape(nz, ny, nx))
+    assert np.array_equal(got[0], got[1])
+    d = a.numpy().astype(np.complex128).reshape(nz, ny, nx)
+    want = np.exp(-1j * (2 * np.pi / .5 * .1) * d)
+    if kind != "c64" and absorb:
+        want = want * bpm_ref.taper_f32(nx, ny, absorb).astype(np.float64)
+    assert np.abs(got[0] - want).max() < 3e-7
