@@ -509,10 +509,13 @@ struct Voxel {
   float u;
   float2 ex, ey, ez;
 };
-__device__ __forceinline__ Voxel octant_sample(int ix, int jy, int kz, int nxo, int M, int Zo, float ex0, float ey0,
-                                               const float2* __restrict__ I, const float* __restrict__ trig) {
+__device__ __forceinline__ Voxel octant_sample(int ix, int jy, int kz, int nxo, int M, int Mr, int Zo, float ex0,
+                                               float ey0, const float2* __restrict__ I,
+                                               const float* __restrict__ trig) {
   const int m = jy * nxo + ix;
-  const size_t ZM = (size_t)Zo * M, o = (size_t)kz * M + m;
+  // the sample's radius row: with a symmetric octant (Mr < M) the pair (min, max) in triangular order
+  const int hi = max(ix, jy), row = Mr < M ? hi * (hi + 1) / 2 + min(ix, jy) : m;
+  const size_t ZM = (size_t)Zo * Mr, o = (size_t)kz * Mr + row;
   const float2 I0 = __ldg(I + o), I1 = __ldg(I + ZM + o), I2 = __ldg(I + 2 * ZM + o);
   const float c1 = __ldg(trig + m), s1 = __ldg(trig + M + m);
   const float c2 = __ldg(trig + 2 * M + m), s2 = __ldg(trig + 3 * M + m);
@@ -529,7 +532,7 @@ __device__ __forceinline__ Voxel octant_sample(int ix, int jy, int kz, int nxo, 
 // (conjugated fields where MIR_STD asks for it)
 template <int MIR>
 __device__ __forceinline__ Voxel assemble_point(int x, int y, int z, int nx, int ny, int nz, const OctGeom& g, int M,
-                                                int Zo, float ex0, float ey0, const float2* __restrict__ I,
+                                                int Mr, int Zo, float ex0, float ey0, const float2* __restrict__ I,
                                                 const float* __restrict__ trig) {
   int ix, jy, kz;
   bool conj;
@@ -542,7 +545,7 @@ __device__ __forceinline__ Voxel assemble_point(int x, int y, int z, int nx, int
     kz = z >= nz - g.nzo ? z - (nz - g.nzo) : g.nzo - 1 - z;
     conj = false;
   }
-  Voxel r = octant_sample(ix, jy, kz, g.nxo, M, Zo, ex0, ey0, I, trig);
+  Voxel r = octant_sample(ix, jy, kz, g.nxo, M, Mr, Zo, ex0, ey0, I, trig);
   if (conj) {
     r.ex.y = -r.ex.y;
     r.ey.y = -r.ey.y;
@@ -556,7 +559,7 @@ __device__ __forceinline__ Voxel assemble_point(int x, int y, int z, int nx, int
 // stores beat the scatter form's single ones; each sample is read by every voxel mirroring
 // onto it
 template <int MIR>
-__global__ void debye_assemble_kernel(int nx, int ny, int nz, OctGeom g, int M, int Zo, float ex0, float ey0,
+__global__ void debye_assemble_kernel(int nx, int ny, int nz, OctGeom g, int M, int Mr, int Zo, float ex0, float ey0,
                                       const float2* __restrict__ I, const float* __restrict__ trig,
                                       float* __restrict__ u, float2* __restrict__ ex, float2* __restrict__ ey,
                                       float2* __restrict__ ez) {
@@ -564,8 +567,8 @@ __global__ void debye_assemble_kernel(int nx, int ny, int nz, OctGeom g, int M, 
   const int x = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (x >= nx) return;
   dep_wait();
-  const Voxel a = assemble_point<MIR>(x, y, z, nx, ny, nz, g, M, Zo, ex0, ey0, I, trig);
-  const Voxel b = assemble_point<MIR>(x + 1, y, z, nx, ny, nz, g, M, Zo, ex0, ey0, I, trig);
+  const Voxel a = assemble_point<MIR>(x, y, z, nx, ny, nz, g, M, Mr, Zo, ex0, ey0, I, trig);
+  const Voxel b = assemble_point<MIR>(x + 1, y, z, nx, ny, nz, g, M, Mr, Zo, ex0, ey0, I, trig);
   const size_t v = ((size_t)z * ny + y) * nx + x;  // even: 8-byte u pairs, 16-byte field pairs
   if (u) __stcs(reinterpret_cast<float2*>(u + v), make_float2(a.u, b.u));
   if (ex) __stcs(reinterpret_cast<float4*>(ex + v), make_float4(a.ex.x, a.ex.y, b.ex.x, b.ex.y));
@@ -599,19 +602,19 @@ __device__ __forceinline__ int mirror_positions(int q, int N0, int N, int (&p)[2
 // sample instead of once per voxel (an 8-fold cut of the reads, the whole cost of an
 // intensity-only call).
 template <int MIR, bool FIELDS>
-__global__ void debye_scatter_kernel(int nx, int ny, int nz, OctGeom g, int M, int Zo, float ex0, float ey0,
+__global__ void debye_scatter_kernel(int nx, int ny, int nz, OctGeom g, int M, int Mr, int Zo, float ex0, float ey0,
                                      const float2* __restrict__ I, const float* __restrict__ trig,
                                      float* __restrict__ u, float2* __restrict__ ex, float2* __restrict__ ey,
                                      float2* __restrict__ ez) {
-  const int ix = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y, kz = blockIdx.z;
-  if (ix >= g.nxo) return;
+  const int ix = blockIdx.x * blockDim.x + threadIdx.x, jy = blockIdx.y * blockDim.y + threadIdx.y, kz = blockIdx.z;
+  if (ix >= g.nxo || jy >= g.nyo) return;
   int px[2], py[2], pz[2];
   const int nxp = mirror_positions<MIR>(ix, nx, g.nxo, px);
   const int nyp = mirror_positions<MIR>(jy, ny, g.nyo, py);
   const int nzp = mirror_positions<MIR>(kz, nz, g.nzo, pz);
   if (nxp == 0 || nyp == 0 || nzp == 0) return;
   dep_wait();
-  const Voxel v = octant_sample(ix, jy, kz, g.nxo, M, Zo, ex0, ey0, I, trig);
+  const Voxel v = octant_sample(ix, jy, kz, g.nxo, M, Mr, Zo, ex0, ey0, I, trig);
 #pragma unroll
   for (int c = 0; c < 2; c++) {
     if (c >= nzp) break;
@@ -643,27 +646,30 @@ __global__ void debye_scatter_kernel(int nx, int ny, int nz, OctGeom g, int M, i
 }
 
 // launch the assembly: the paired gather form when fields are written to 16-byte aligned
-// buffers of even nx (GB300, 256^3 with all four outputs: gather 82 us against 90 us for the
-// scatter form), else one thread per octant sample (intensity only: 0.172 -> 0.151 ms for the
-// whole 256^3 PSF)
-int launch_assemble(const debye_desc* d, bool gauss, const OctGeom& g, int M, int Zo, const float2* I,
+// buffers of even nx and every octant column has its own radius row (GB300, 256^3 with all four
+// outputs: 82 us against 90 for the scatter form), else one thread per octant sample. With a
+// symmetric octant the samples past the diagonal lie in columns of the triangular rows: gathered
+// by all of their voxels that took 124 us. Scatter blocks are 32 threads along x by 4 along y, so
+// four neighbouring y share the 32 bytes that a warp fetches for one.
+int launch_assemble(const debye_desc* d, bool gauss, const OctGeom& g, int M, int Mr, int Zo, const float2* I,
                     const float* trig, float* u, void* ex, void* ey, void* ez, cudaStream_t s) {
   float2 *pex = static_cast<float2*>(ex), *pey = static_cast<float2*>(ey), *pez = static_cast<float2*>(ez);
   const float e0 = (float)d->ex0, e1 = (float)d->ey0;
   const bool fields = ex || ey || ez;
   const bool pair = d->nx % 2 == 0 && ((uintptr_t)u & 7) == 0 && ((uintptr_t)ex & 15) == 0 &&
                     ((uintptr_t)ey & 15) == 0 && ((uintptr_t)ez & 15) == 0;
-  if (fields && pair) {
+  if (fields && pair && Mr == M) {
     const dim3 grid((d->nx / 2 + 127) / 128, d->ny, d->nz);
-    BPM_CUDA_TRY(launch_dep(gauss ? debye_assemble_kernel<MIR_GAUSS> : debye_assemble_kernel<MIR_STD>, grid, dim3(128),
-                            0, s, d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex, pey, pez));
+    BPM_CUDA_TRY(launch_dep(gauss ? debye_assemble_kernel<MIR_GAUSS> : debye_assemble_kernel<MIR_STD>, grid,
+                            dim3(128), 0, s, d->nx, d->ny, d->nz, g, M, Mr, Zo, e0, e1, I, trig, u, pex, pey, pez));
     BPM_LAUNCH_CHECK("debye_assemble_kernel");
     return BPM_OK;
   }
-  const dim3 grid((g.nxo + 127) / 128, g.nyo, g.nzo);
+  const dim3 grid((g.nxo + 31) / 32, (g.nyo + 3) / 4, g.nzo);
   auto fn = gauss ? (fields ? debye_scatter_kernel<MIR_GAUSS, true> : debye_scatter_kernel<MIR_GAUSS, false>)
                   : (fields ? debye_scatter_kernel<MIR_STD, true> : debye_scatter_kernel<MIR_STD, false>);
-  BPM_CUDA_TRY(launch_dep(fn, grid, dim3(128), 0, s, d->nx, d->ny, d->nz, g, M, Zo, e0, e1, I, trig, u, pex, pey, pez));
+  BPM_CUDA_TRY(launch_dep(fn, grid, dim3(32, 4), 0, s, d->nx, d->ny, d->nz, g, M, Mr, Zo, e0, e1, I, trig, u, pex, pey,
+                          pez));
   BPM_LAUNCH_CHECK("debye_scatter_kernel");
   return BPM_OK;
 }
@@ -944,8 +950,7 @@ struct TcArgs {
   uint32_t tmem_cols;
   int nacc;        // accumulators in tensor memory (2 or 3), acc_stride columns apart
   int acc_stride;
-  int nxo, M, sym; // octant columns per row, octant columns, radius rows deduplicated
-  float2* I;       // (3, Zo, M): row r of the product goes to its octant column(s)
+  float2* I;       // (3, Zo, Mr)
   unsigned long long wait_ns;  // limit of every mbarrier wait
   unsigned extra_tx;           // 0; debye_tc_timeout_selftest announces bytes that never arrive
 };
@@ -1093,12 +1098,7 @@ debye_accum_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     const int row = m0 + warp * 32 + lane;
     const bool rv = row < a.rows;
     const int n = rv ? row / a.Mr : 0, r = rv ? row - n * a.Mr : 0;
-    // octant column (ix, jy) of the row and, for a deduplicated row off the diagonal, its
-    // mirror (jy, ix): both receive the integrals, so I keeps the plain column layout
-    const int m1 = radius_column(r, a.nxo, a.sym != 0);
-    const int ix = m1 % a.nxo, jy = m1 / a.nxo;
-    const int m2 = (a.sym && ix != jy) ? ix * a.nxo + jy : -1;
-    const size_t ob = ((size_t)n * a.Zo) * a.M;
+    float2* out = a.I + (size_t)n * a.Zo * a.Mr + r;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
     const bool two_big = a.nacc == 3 && KT > 1;  // the odd-slice accumulator was written
     for (int c0 = 0; c0 < a.BN; c0 += 16) {
@@ -1116,11 +1116,7 @@ debye_accum_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           const int z = (n0 + c0) / 2 + j;
-          if (z < a.Zo) {
-            const float2 val = make_float2(v[2 * j], v[2 * j + 1]);
-            a.I[ob + (size_t)z * a.M + m1] = val;
-            if (m2 >= 0) a.I[ob + (size_t)z * a.M + m2] = val;
-          }
+          if (z < a.Zo) out[(size_t)z * a.Mr] = make_float2(v[2 * j], v[2 * j + 1]);
         }
       }
     }
@@ -1314,7 +1310,7 @@ TcLayout tc_layout(const debye_desc* d, bool gauss) {
   L.A = off; off += align256(sizeof(float) * 3 * (size_t)L.Mr * L.Tp);
   L.Bh = off; off += align256(sizeof(float) * 2 * (size_t)L.Zo * L.Tp);
   L.Bl = off; off += align256(sizeof(float) * 2 * (size_t)L.Zo * L.Tp);
-  L.I = off; off += align256(sizeof(float2) * 3 * (size_t)L.Zo * L.M);
+  L.I = off; off += align256(sizeof(float2) * 3 * (size_t)L.Zo * L.Mr);
   L.total = off;
   return L;
 }
@@ -1380,9 +1376,6 @@ int run_octant_tc(const debye_desc* d, bool gauss, double sig, float* u, void* e
     while (c < need) c <<= 1;
     ta.tmem_cols = c;
   }
-  ta.nxo = L.nxo;
-  ta.M = L.M;
-  ta.sym = L.sym ? 1 : 0;
   ta.I = I;
   ta.wait_ns = TC_WAIT_NS;
   ta.extra_tx = 0;
@@ -1392,7 +1385,7 @@ int run_octant_tc(const debye_desc* d, bool gauss, double sig, float* u, void* e
   const dim3 grid(L.ntn, (rows + TC_BM - 1) / TC_BM);
   BPM_CUDA_TRY(launch_dep(debye_accum_tc_kernel, grid, dim3(TC_THREADS), smem, s, mA, mBh, mBl, ta));
   BPM_LAUNCH_CHECK("debye_accum_tc_kernel");
-  if (u || ex || ey || ez) return launch_assemble(d, gauss, g, L.M, L.Zo, I, trig, u, ex, ey, ez, s);
+  if (u || ex || ey || ez) return launch_assemble(d, gauss, g, L.M, L.Mr, L.Zo, I, trig, u, ex, ey, ez, s);
   return BPM_OK;
 }
 
@@ -1445,7 +1438,7 @@ int run_octant(const debye_desc* d, bool gauss, double sig, float* u, void* ex, 
     debye_accum_rem_kernel<1><<<rtiles, 256, 0, s>>>(L.T, L.M, L.Mp, L.Zo, L.Zp, nrz, J, E, I);
     BPM_LAUNCH_CHECK("debye_accum_rem_kernel");
   }
-  if (u || ex || ey || ez) return launch_assemble(d, gauss, g, L.M, L.Zo, I, trig, u, ex, ey, ez, s);
+  if (u || ex || ey || ez) return launch_assemble(d, gauss, g, L.M, L.M, L.Zo, I, trig, u, ex, ey, ez, s);
   return BPM_OK;
 }
 
@@ -1632,9 +1625,6 @@ extern "C" int debye_tc_timeout_selftest(double wait_ms) {
   ta.acc_stride = 32;
   ta.nacc = 3;
   ta.tmem_cols = 128;
-  ta.nxo = rows;
-  ta.M = rows;
-  ta.sym = 0;
   ta.I = I;
   ta.wait_ns = (unsigned long long)(wait_ms * 1e6);
   ta.extra_tx = 16;
