@@ -849,23 +849,11 @@ __device__ int g_tc_status;  // nonzero once a tensor-core wait gave up (bpm_dev
 
 __device__ __forceinline__ float tf32_hi(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
 
-// octant column jy * nxo + ix of radius row r: with a symmetric octant (the x and y grids
-// equal) the rows are the distinct pairs ix <= jy in triangular order r = jy (jy + 1) / 2 + ix,
-// else r is the column itself
-__device__ __forceinline__ int radius_column(int r, int nxo, bool sym) {
-  if (!sym) return r;
-  int b = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * .5f);
-  while (b * (b + 1) / 2 > r) b--;
-  while ((b + 1) * (b + 2) / 2 <= r) b++;
-  const int a = r - b * (b + 1) / 2;
-  return b * nxo + a;
-}
-
 // Nodes and radii of the tensor-core path in one launch: blocks [0, nbn) one quadrature node
 // per thread (as debye_nodes_kernel: cos t in FP64 for the phases, the three node factors,
 // sin t as a float pair), the others one octant column per thread (as debye_radii_kernel,
 // k r as a float pair). 32-thread blocks spread the FP64 chains over the SMs.
-__global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, int M, int nbn, double* ct,
+__global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, int M, int sym, int nbn, double* ct,
                                       float* wf, float2* si2, float2* kr2, float* trig) {
   dep_release();
   if ((int)blockIdx.x < nbn) {
@@ -880,8 +868,14 @@ __global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, in
     const int m = (blockIdx.x - nbn) * blockDim.x + threadIdx.x;
     if (m >= M) return;
     float4 tv;
-    kr2[m] = split_pair(radius_values(g, k, m, tv));
+    const float2 kr = split_pair(radius_values(g, k, m, tv));
     trig_store(trig, M, m, tv);
+    // k r by radius row: with a symmetric octant the distinct pairs ix <= jy in triangular order
+    const int jy = m / g.nxo, ix = m - jy * g.nxo;
+    if (!sym)
+      kr2[m] = kr;
+    else if (ix <= jy)
+      kr2[jy * (jy + 1) / 2 + ix] = kr;
   }
 }
 
@@ -894,7 +888,7 @@ __global__ void debye_setup_tc_kernel(NodeArgs a, OctGeom g, double k, int T, in
 // A Bessel evaluation is about 65 instructions, so with one row a block the device spent the
 // launch placing blocks (42 570 of them at 256^3): up to 8 rows a block share the node's values.
 __global__ void __launch_bounds__(128) debye_tables_tc_kernel(
-    int T, int Tp, int Mr, int nxo, int sym, int Zo, int rpb, float z1, float z2, double k,
+    int T, int Tp, int Mr, int Zo, int rpb, float z1, float z2, double k,
     const double* __restrict__ ct, const float2* __restrict__ si2, const float2* __restrict__ kr2,
     const float* __restrict__ wf, float* __restrict__ A, float* __restrict__ Bh, float* __restrict__ Bl) {
   const int t = blockIdx.y * 128 + threadIdx.x;
@@ -921,7 +915,7 @@ __global__ void __launch_bounds__(128) debye_tables_tc_kernel(
 #pragma unroll 2
   for (int row = max(row0, Zo); row < row1; row++) {
     const int r = row - Zo;
-    const float x = mul_pair(kr2[radius_column(r, nxo, sym != 0)], sv);
+    const float x = mul_pair(kr2[r], sv);
     float j0, j1, j2;
     bessel_j012(x, j0, j1, j2);
     float* o = A + (size_t)r * Tp + t;
@@ -1075,8 +1069,10 @@ debye_accum_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
       const uint32_t sa = tc::smem_u32(sm + (size_t)st * SB), sl = sa + AB, sbh = sa + 2 * AB, sbl = sbh + BB;
       const uint32_t big = a.nacc == 3 ? tmem + (uint32_t)((kt & 1) * a.acc_stride) : tmem;
       const uint32_t cross = tmem + (uint32_t)((a.nacc - 1) * a.acc_stride);
+      const int steps = min(TC_BK, a.T - kt * TC_BK + 7) / 8;  // the last slice: as far as it has nodes
 #pragma unroll
       for (int k = 0; k < TC_BK / 8; k++) {  // 8 TF32 (32 bytes) of K per instruction
+        if (k >= steps) break;
         const uint64_t dah = tc::desc_sw128_kmajor(sa + 32 * k), dal = tc::desc_sw128_kmajor(sl + 32 * k);
         const uint64_t dbh = tc::desc_sw128_kmajor(sbh + 32 * k), dbl = tc::desc_sw128_kmajor(sbl + 32 * k);
         const bool first_big = a.nacc == 3 ? (kt < 2 && k == 0) : (kt == 0 && k == 0);
@@ -1352,13 +1348,13 @@ int run_octant_tc(const debye_desc* d, bool gauss, double sig, float* u, void* e
   }
   const int tb = (L.T + 127) / 128;
   const int nbn = (L.T + 31) / 32;
-  debye_setup_tc_kernel<<<(unsigned)(nbn + (L.M + 31) / 32), 32, 0, s>>>(na, g, k, L.T, L.M, nbn, ct, wf, si2, kr2,
-                                                                          trig);
+  debye_setup_tc_kernel<<<(unsigned)(nbn + (L.M + 31) / 32), 32, 0, s>>>(
+      na, g, k, L.T, L.M, L.sym ? 1 : 0, nbn, ct, wf, si2, kr2, trig);
   BPM_LAUNCH_CHECK("debye_setup_tc_kernel");
   // rows per block: blocks for a few waves of 16 on each of 152 SMs
   const int rpb = (int)std::min<long long>(8, std::max<long long>(1, (long long)(L.Zo + L.Mr) * tb / (152 * 64)));
   BPM_CUDA_TRY(launch_dep(debye_tables_tc_kernel, dim3((unsigned)((L.Zo + L.Mr + rpb - 1) / rpb), (unsigned)tb),
-                          dim3(128), 0, s, L.T, L.Tp, L.Mr, L.nxo, L.sym ? 1 : 0, L.Zo, rpb, g.z1, g.z2, k,
+                          dim3(128), 0, s, L.T, L.Tp, L.Mr, L.Zo, rpb, g.z1, g.z2, k,
                           (const double*)ct, (const float2*)si2, (const float2*)kr2, (const float*)wf, A, Bh, Bl));
   BPM_LAUNCH_CHECK("debye_tables_tc_kernel");
   TcArgs ta;
