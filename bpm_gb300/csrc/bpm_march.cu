@@ -1877,12 +1877,25 @@ void prepare_kernels(int nx, int ny) {
   }
 }
 
-int default_group(const bpm_plan* pl, int batch) {
+// Fields per group of a march whose groups follow one another (the adjoint): planes of 16 MB, so
+// that a group stays resident in the 129 MB L2 next to the dn slices and output streams
+int serial_group(const bpm_plan* pl, int batch) {
   const size_t plane_bytes = (size_t)pl->d.nx * pl->d.ny * 8;
-  // up to kMaxConcurrentGroups groups march at once: keep each group's planes near 16 MB so
-  // all of them stay resident in the 129 MB L2 next to the dn slices and output streams
   const int g = (int)std::max<size_t>(1, (16u << 20) / plane_bytes);
   return std::max(1, std::min(g, batch));
+}
+
+// ... and of one whose groups march at once, up to kMaxConcurrentGroups of them. From 12 MB of
+// planes on, fields of up to 1 MB go in at least two groups of even size, so that one's loads and
+// block launches run beside the other's arithmetic (GB300, us per step without the sums: 32 fields
+// of 256^2 22.5 -> 18.2, 24 of them 18.3 -> 15.0, 16 of 512 x 256 23.4 -> 20.6, 24 of 512 x 128
+// 21.6 -> 18.5; 16 of 256^2, 8 MB, are 4 % slower in two groups, and so are 8 of 512^2).
+int default_group(const bpm_plan* pl, int batch) {
+  const size_t plane_bytes = (size_t)pl->d.nx * pl->d.ny * 8;
+  const int g = serial_group(pl, batch);
+  if (plane_bytes > (1u << 20) || plane_bytes * batch < (12u << 20)) return g;
+  const int groups = std::max(2, (batch + g - 1) / g);
+  return (batch + groups - 1) / groups;
 }
 
 struct WsLayout {
@@ -1975,10 +1988,11 @@ int check_workspace(const bpm_plan* pl, const bpm_request* r, const void* ws, si
   return BPM_OK;
 }
 
-MarchCtx make_ctx(const bpm_plan* pl, const bpm_request* r, void* ws, int b0, int Gc) {
+// of a workspace slot laid out for groups of G fields
+MarchCtx make_ctx(const bpm_plan* pl, const bpm_request* r, void* ws, int b0, int Gc, int G) {
   const bpm_grid_desc& d = pl->d;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  WsLayout L = ws_layout(pl, group_size(pl, r));
+  WsLayout L = ws_layout(pl, G);
   char* wsb = static_cast<char*>(ws);
   float2* W = reinterpret_cast<float2*>(wsb + L.w);
   float* red = reinterpret_cast<float*>(wsb + L.red);
@@ -2219,7 +2233,7 @@ struct ClusterK {
     }) == 1;
   }
   static int launch(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
-    MarchCtx c = make_ctx(pl, r, ws, 0, r->batch);
+    MarchCtx c = make_ctx(pl, r, ws, 0, r->batch, group_size(pl, r));
     ClusterArgs a;
     a.rp = c.rp;
     a.rp.do_mask = r->dn_dtype != BPM_DN_NONE;
@@ -2287,7 +2301,7 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
     return kNotGrid;
   const int G = group_size(pl, r);
   if (G < r->batch || r->batch > grid_march_capacity(d.nx, d.ny)) return kNotGrid;
-  MarchCtx c = make_ctx(pl, r, ws, 0, r->batch);
+  MarchCtx c = make_ctx(pl, r, ws, 0, r->batch, G);
   GridMarchArgs a;
   a.rp = c.rp;
   a.rp.do_mask = r->dn_dtype != BPM_DN_NONE;
@@ -2298,6 +2312,8 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
   a.wait_ns = kMarchWaitNs;
   return grid_march_launch(d.nx, d.ny, a, r->batch, s);
 }
+
+std::recursive_mutex g_aux_mu;
 
 // All groups of a request. With room for several workspace slots, groups march
 // concurrently on the plan's auxiliary streams (forked from and joined back to s through
@@ -2339,6 +2355,10 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   const size_t slot = ws_layout(pl, G).total;
   const int conc = std::max(
       1, (int)std::min<size_t>({(size_t)ngroups, ws_bytes / slot, (size_t)(r->conc > 0 ? r->conc : conc_limit())}));
+  // the plan's streams and events are shared by every caller of the plan: one at a time hands
+  // them work, so that no caller's fork or join takes another's event
+  std::unique_lock<std::recursive_mutex> lock(g_aux_mu, std::defer_lock);
+  if (conc > 1 || sink) lock.lock();
   cudaStream_t st[kMaxConcurrentGroups];
   for (int j = 0; j < conc; j++) st[j] = conc > 1 ? pl->aux[j] : s;
   if (conc > 1 || sink) BPM_CUDA_TRY(cudaEventRecord(pl->ev_fork, s));
@@ -2354,7 +2374,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
       b0[j] = (w0 + j) * G;
       Gc[j] = std::min(G, r->batch - b0[j]);
       zdone[j] = 0;
-      c[j] = make_ctx(pl, r, static_cast<char*>(ws) + (size_t)j * slot, b0[j], Gc[j]);
+      c[j] = make_ctx(pl, r, static_cast<char*>(ws) + (size_t)j * slot, b0[j], Gc[j], G);
       if (j == 0)
         pp = plan_passes(d.nx, r->batch, nwave, [&] {
           int e = launch_first_row(pl, r, c[0], b0[0], st[0]);
@@ -2460,7 +2480,7 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
                      void* ws, size_t ws_bytes, cudaStream_t s) {
   const bpm_grid_desc& d = pl->d;
   const int nz = d.nz, k = r->ckpt_every;
-  const int G = group_size(pl, r);
+  const int G = r->group > 0 ? std::min(r->group, r->batch) : serial_group(pl, r->batch);
   BwLayout L = bw_layout(pl, G, k);
   if (!ws || ws_bytes < L.total || ((uintptr_t)ws & 15)) {
     set_error("workspace too small or misaligned: need " + std::to_string(L.total) + " bytes");
@@ -2477,7 +2497,7 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
   for (int b0 = 0; b0 < r->batch; b0 += G) {
     const int Gc = std::min(G, r->batch - b0);
     // forward recompute context on its own workspace, writing fields into the segment buffer
-    MarchCtx cf = make_ctx(pl, r, wsb + L.fwd, b0, Gc);
+    MarchCtx cf = make_ctx(pl, r, wsb + L.fwd, b0, Gc, G);
     cf.rp.out = seg;
     cf.rp.out_kind = BPM_OUT_FIELD;
     cf.rp.out_bstride = (long long)(k + 1) * plane;
@@ -2486,7 +2506,7 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
     cf.rp.scat_p = cf.rp.scat_g = nullptr;
     cf.cp.scat = 0;
     // adjoint context
-    MarchCtx ca = make_ctx(pl, r, wsb + L.adj, b0, Gc);
+    MarchCtx ca = make_ctx(pl, r, wsb + L.adj, b0, Gc, G);
     ca.rp.out = nullptr;
     ca.rp.out_kind = BPM_OUT_NONE;
     ca.rp.last_plane = nullptr;
@@ -2836,7 +2856,7 @@ extern "C" int bpm_launch_pass(bpm_plan* pl, const bpm_request* r, void* ws, siz
   if ((rc = check_workspace(pl, r, ws, ws_bytes))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int Gc = group_size(pl, r);
-  MarchCtx c = make_ctx(pl, r, ws, 0, Gc);
+  MarchCtx c = make_ctx(pl, r, ws, 0, Gc, Gc);
   switch (pass) {
     case BPM_PASS_FIRST_ROW:
       return launch_first_row(pl, r, c, 0, s);
@@ -2862,7 +2882,7 @@ extern "C" int bpm_launch_pass(bpm_plan* pl, const bpm_request* r, void* ws, siz
 
 extern "C" size_t bpm_backward_workspace_bytes(const bpm_plan* pl, int batch, int group, int ckpt_every) {
   if (!pl || batch < 1 || ckpt_every < 1) return 0;
-  const int G = group > 0 ? std::min(group, batch) : default_group(pl, batch);
+  const int G = group > 0 ? std::min(group, batch) : serial_group(pl, batch);
   return bw_layout(pl, G, ckpt_every).total;
 }
 
@@ -2914,6 +2934,7 @@ extern "C" int bpm_exec_create(bpm_plan* pl, const bpm_request* r, void* ws, siz
   if (!pl || !out) { set_error("plan/out is NULL"); return BPM_ERR_ARG; }
   int rc = check_request(pl, r);
   if (rc) return rc;
+  std::lock_guard<std::recursive_mutex> lock(g_aux_mu);  // the plan's streams join the capture
   cudaStream_t s;
   BPM_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   unsigned long long before = g_launches.load();

@@ -650,3 +650,26 @@ def test_mask_precompute_aligned_and_unaligned(bpm, kind, size, absorb):
     if kind != "c64" and absorb:
         want = want * bpm_ref.taper_f32(nx, ny, absorb).astype(np.float64)
     assert np.abs(got[0] - want).max() < 3e-7
+
+
+@pytest.mark.parametrize("size,mode,batch", [((256, 256, 4), "weighted", 25), ((512, 128, 4), "ignore", 24),
+                                             ((128, 512, 3), "simple", 33)])
+def test_batches_in_two_groups_equal_single_fields(bpm, size, mode, batch):
+    """Batches that the library splits into concurrent groups of its own accord (odd remainders
+    included), also as a captured graph: each field equals the field marched alone, bit for bit."""
+    import torch
+    Nx, Ny, Nz = size
+    rng = np.random.default_rng(batch)
+    dn = torch.from_numpy((.03 * rng.standard_normal((Nz, Ny, Nx))).astype(np.float32)).cuda()
+    x = .1 * np.arange(Nx)
+    u0 = np.exp(2j * np.pi * rng.uniform(-.3, .3, (batch, 1, 1)) * x[None, None, :]).repeat(Ny, 1)
+    u0 = torch.from_numpy(u0.astype(np.complex64)).cuda()
+    kw = dict(lam=.5, n0=1.33, dn=dn, mean_mode=mode, return_field=False)
+    got = bpm.bpm_3d_batched(size, (.1, .1, .1), u0=u0, **kw)
+    m = bpm.BatchedMarch(size, (.1, .1, .1), .5, 1.33, batch, dn=dn, mean_mode=mode)
+    m.u0.copy_(u0)
+    m.run()
+    torch.cuda.synchronize()
+    assert m.group_used < batch and torch.equal(m.out, got)
+    for b in (0, batch // 2, batch - 1):
+        assert torch.equal(got[b], bpm.bpm_3d(size, (.1, .1, .1), u0=u0[b], **kw)), b
