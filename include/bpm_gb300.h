@@ -110,7 +110,11 @@ typedef struct {
   int col_block;                 /* columns per block of the non-weighted column passes, 4, 8 or 16 */
   int cluster;                   /* whole-march cluster kernel (square 64..256 grids without
                                     scattering sums or checkpoints): 1 = use it, 2 = row/column
-                                    pass kernels (default: cluster at 64)                       */
+                                    pass kernels only, for requests that march beside others.
+                                    Default: the cluster kernel at 64, at 128 but for large
+                                    batches without the weighted sums, and for 3 or 4 weighted
+                                    fields of 256; one cooperative launch for one or a few
+                                    fields of other grids from 128 up; else pass kernels        */
   int col_fuse;                  /* weighted mode: 1 = one column pass per step (forward FFT,
                                     plane-wide sums across a thread-block cluster of the field's
                                     blocks, propagator, inverse FFT) where ny <= 512, nx <= 512
@@ -313,9 +317,10 @@ typedef struct {
 /* Bytes of scratch debye_focus_field needs for this description (256-aligned). */
 size_t debye_workspace_bytes(const debye_desc* desc);
 
-/* Sticky device-side status of the tensor-core kernels: nonzero once one of their bounded
- * waits (an mbarrier that a TMA copy or a tensor-core product should complete) gave up
- * after 2 s, in which case that launch left its outputs unwritten. Synchronises with the
+/* Sticky device-side status of the kernels with bounded waits: nonzero once one of the
+ * tensor-core quadrature's (an mbarrier that a TMA copy or a tensor-core product should
+ * complete) or one of the whole-march kernels' (tiles or arrivals of the field's other blocks)
+ * gave up after 2 s, in which case that launch left its outputs unwritten or wrong. Synchronises with the
  * device to read it; clear != 0 resets it to 0. A negative bpm_status on a CUDA error.
  * No counterpart in the reference (its OpenCL kernels have no such waits). */
 int bpm_device_status(int clear);
