@@ -32,7 +32,7 @@ from . import _native as N
 __all__ = ["tune_shape", "tune_group", "pick_group", "pick_option", "shape_candidates", "cache_path"]
 
 _cache = None
-_VERSION = 4  # cache entries of another layout are measured again
+_VERSION = 5  # cache entries of another layout, or of other kernels, are measured again
 
 
 def cache_path():

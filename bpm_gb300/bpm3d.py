@@ -675,13 +675,16 @@ class MixedBatch:
             shape = (B, Nz, Ny, Nx)
             out = torch.empty(shape, dtype=torch.complex64 if ok == N.OUT_FIELD else torch.float32, device=dev)
             last = torch.empty((B, Ny, Nx), dtype=torch.complex64, device=dev)
-            # groups march beside one another: pass kernels, which interleave (the one-launch
-            # march of a few fields would hold its part of every SM until it ends)
-            launch = {"cluster": 2} if len(groups) > 1 and min(Nx, Ny) >= 128 and (Nx, Ny) != (128, 128) else {}
+            launch = {}
             if tune:
                 from .autotune import tune_shape
                 launch = tune_shape((Nx, Ny, Nz), r0.units, r0.lam, r0.n0, B, dn, r0.mean_mode, out_kind,
                                     r0.absorbing_width)
+            # groups march beside one another: pass kernels, which interleave, whatever is the faster
+            # for a group alone (a whole-march kernel holds its part of every SM until it ends; at
+            # 64^2 and 128^2 it takes few SMs)
+            if len(groups) > 1 and (Nx, Ny) not in ((64, 64), (128, 128)):
+                launch = dict(launch, cluster=2)
             wsb = plan.workspace_bytes(B, launch.get("group", 0), launch.get("conc", 0))
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
             req = N.Request(B, _ptr(u0), _ptr(dn), kind, 0, None, None, _ptr(out), ok, Nz * Ny * Nx, _ptr(last),

@@ -1554,12 +1554,15 @@ int pass_launch(const char* what, int carve, void (*kernel)(KArgs...), dim3 grid
 // registers and threads let them be resident together. The largest partition, with the L1 cache at
 // its smallest, makes the 512^2 batches 3 % slower. A single field of 1024 columns, whose row
 // blocks hold twice the registers, takes the driver's choice (1024 x 256 9.9 against 12.7).
+// beside: the request says that it marches beside others (cluster = 2). Their passes share the SMs,
+// and a block that asks for another partition waits until an SM is idle: 48 marches of 128^2, 256^2
+// and 512^2 as branches of one graph take 10.3 ms with a partition per march and 9.4 with none.
 struct PassPlan {
   int carve, early;
 };
 template <class F>
-PassPlan plan_passes(int nx, int fields, int conc, F passes) {
-  if (fields == 1 && nx == 1024) return {0, 1};
+PassPlan plan_passes(int nx, int fields, bool beside, int conc, F passes) {
+  if (beside || (fields == 1 && nx == 1024)) return {0, 1};
   PassNeed need{(size_t)conc, 0, {}, {}};
   t_need = &need;
   const int rc = passes();
@@ -2376,7 +2379,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
       zdone[j] = 0;
       c[j] = make_ctx(pl, r, static_cast<char*>(ws) + (size_t)j * slot, b0[j], Gc[j], G);
       if (j == 0)
-        pp = plan_passes(d.nx, r->batch, nwave, [&] {
+        pp = plan_passes(d.nx, r->batch, r->cluster == 2, nwave, [&] {
           int e = launch_first_row(pl, r, c[0], b0[0], st[0]);
           if (!e && nz > 1) e = launch_cols(pl, c[0], 0, 0, st[0]);
           return e || nz == 1 ? e : launch_row_z(pl, r, c[0], 1, st[0]);
@@ -2528,7 +2531,7 @@ int enqueue_backward(bpm_plan* pl, const bpm_request* r, const void* grad_last, 
       ca.rp.seg = ck;
       ca.rp.seg_bstride = (long long)n_ckpt * plane;
     }
-    const PassPlan pp = plan_passes(d.nx, r->batch, 1, [&] {
+    const PassPlan pp = plan_passes(d.nx, r->batch, r->cluster == 2, 1, [&] {
       RowParams m = ca.rp;
       m.z = 1;
       m.do_inv = m.do_fwd = 1;

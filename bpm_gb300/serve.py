@@ -355,11 +355,12 @@ class Server:
         ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
         req = N.Request(B, _ptr(u0), _ptr(dn), kind, dn_stride, None, None,
                         _ptr(out), ok, Nz * Ny * Nx, _ptr(last), None, None, 0, 0, None, 0, _ptr(mask))
-        if Nx == Ny == 128 and self._inflight:
-            # the whole-march cluster kernel, a few SMs per field, beside other launches
-            # whatever the batch (the library's own choice up to 32 fields)
-            req.cluster = 1
-        elif min(Nx, Ny) >= 128:
+        if Nx == Ny == 128:
+            # beside other launches the whole-march cluster kernel, a few SMs per field, whatever
+            # the batch (the library's own choice up to 32 fields)
+            if self._inflight:
+                req.cluster = 1
+        elif (Nx, Ny) != (64, 64):
             # pass kernels, which interleave with the other streams' launches; the library's
             # one-launch march would hold its part of every SM until the march ends
             req.cluster = 2
