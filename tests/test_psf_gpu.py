@@ -316,3 +316,15 @@ def test_assembly_forms_agree(bpm, shape):
     for a, b in zip(gathered, scattered):
         assert torch.equal(a, b)
     assert torch.equal(run(0, fields=False)[0], gathered[0])
+
+
+@pytest.mark.parametrize("nz", [2, 62, 94, 126, 158, 200])
+@pytest.mark.parametrize("steps", [20, 64, 200])
+def test_quadrature_accumulators(bpm, nz, steps):
+    """Tiles of 16 to 208 columns (two to five accumulators) with fewer and more slices of 32
+    nodes than accumulators: a slice added twice, dropped or left from another tile is far off."""
+    args = ((8, 6, nz), (.1, .1, .1), .5, .8, 1.33, steps)
+    out = bpm.focus_field_debye(*args)
+    ref = debye_ref.focus_field_debye(*args, real_dtype=np.float64, complex_dtype=np.complex128)
+    for a, b, k in zip(out, ref, ("u", "ex", "ey", "ez")):
+        assert rel_l2(a, b) < TOL, k
