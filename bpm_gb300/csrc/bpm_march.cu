@@ -1916,9 +1916,11 @@ WsLayout ws_layout(const bpm_plan* pl, int G) {
   L.dn0 = off;
   off += align256((size_t)G * sizeof(float));
   L.scat = off;
-  off += align256((size_t)G * std::max(ntiles, kGridBlocks) * 2 * sizeof(float));
+  // the one-launch march: two copies of its blocks' partial sums, and a counter per field
+  const bool grid = pl->d.nx >= 128 && pl->d.ny >= 128;
+  off += align256((size_t)G * (grid ? 2 * kGridBlocks : ntiles) * 2 * sizeof(float));
   L.counter = off;
-  off += align256((size_t)G * kGridCounterStride * sizeof(unsigned));
+  if (grid) off += align256((size_t)G * kGridCounterStride * sizeof(unsigned));
   L.total = off;
   return L;
 }

@@ -12,8 +12,9 @@
 // the finished plane is written while the team gathers.
 //
 // The blocks of a grid wait on one another, so it is launched cooperatively (every block
-// resident at once) and every wait is bounded in time. FFTs, masks, propagator and sums are
-// those of the pass kernels: the same bits.
+// resident at once) and every wait is bounded in time. FFTs, masks, propagator and weighted sums
+// are those of the pass kernels, so the fields are the same bits; the scattering sums are added
+// per block of C columns, not of 16, and agree to FP32 rounding.
 #include <algorithm>
 #include <string>
 
@@ -81,6 +82,10 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
   const float* sdn = sky2 + NY;
   const int nz = a.nz;
   unsigned* counter = a.counter + gl * kGridCounterStride;
+  // The blocks' partial scattering sums of plane z, two copies by the parity of z: block 0 adds
+  // plane z's behind the gathering of its row phase, when the other blocks may already be storing
+  // those of plane z + 1. They store plane z + 2's only after block 0 has arrived once more.
+  auto scat_part = [&](int z) { return q.scat_part + ((size_t)(2 * gl + (z & 1)) * NB) * 2; };
   unsigned target = 0;
   bool dead = false;
 
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
     if (p.scat_p && b == 0 && warp == 0) {
       float2 s = make_float2(0.f, 0.f);
       if (z > 0) {
-        const float2* part = reinterpret_cast<const float2*>(q.scat_part) + (size_t)gl * NB;
+        const float2* part = reinterpret_cast<const float2*>(scat_part(z));
         for (int k = t; k < NB; k += 32) {
           const float2 w = __ldcg(part + k);
           s.x += w.x;
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
     if (q.scat && tid == 0) {  // red: written before the second transform's barriers
       float S = 0.f, G = 0.f;
       for (int w = 0; w < C; w++) S += red[2 * w], G += red[2 * w + 1];
-      float* o = q.scat_part + ((size_t)gl * NB + b) * 2;
+      float* o = scat_part(z + 1) + 2 * b;
       o[0] = S;
       o[1] = G;
     }

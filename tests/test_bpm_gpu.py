@@ -673,3 +673,25 @@ def test_batches_in_two_groups_equal_single_fields(bpm, size, mode, batch):
     assert m.group_used < batch and torch.equal(m.out, got)
     for b in (0, batch // 2, batch - 1):
         assert torch.equal(got[b], bpm.bpm_3d(size, (.1, .1, .1), u0=u0[b], **kw)), b
+
+
+@pytest.mark.parametrize("size,mode", [((256, 128, 12), "ignore"), ((256, 256, 17), "simple"),
+                                       ((512, 128, 16), "ignore"), ((1024, 256, 9), "simple")])
+def test_one_launch_scattering_sums_stay_with_their_plane(bpm, size, mode):
+    """Without the weighted sums nothing but the two copies of the blocks' partial sums keeps those
+    of neighbouring planes apart: the sums of repeated marches (full field output, which holds the
+    adding block up) are the same bits, and the FP64 oracle's to the parity tolerance, plane by
+    plane from plane 2 on (the sums of neighbouring planes differ by far more)."""
+    Nx, Ny, Nz = size
+    rng = np.random.default_rng(Nx + Nz)
+    dn = (.03 * rng.standard_normal((Nz, Ny, Nx)) * (1 + np.arange(Nz) % 2)[:, None, None]).astype(np.float32)
+    kw = dict(lam=.5, n0=1.33, dn=dn, mean_mode=mode, return_scattering=True, return_g=True)
+    want = bpm_ref.bpm_3d(size, (.1, .1, .1), precision="fp64", **kw)
+    got = [bpm.bpm_3d(size, (.1, .1, .1), **kw)[1:] for _ in range(20)]
+    for p, g in got:
+        assert np.array_equal(p, got[0][0]) and np.array_equal(g[2:], got[0][1][2:])
+    p = want[1]
+    assert np.all(np.abs(p[3:] - p[2:-1]) > 100 * TOL * p[2:-1])
+    for k in (0, 1):  # (nothing has scattered before plane 2: 0 / 0 in g)
+        a, b = got[0][k][2:], np.asarray(want[1 + k])[2:]
+        assert np.all(np.abs(a - b) <= TOL * np.abs(b)), k
