@@ -2339,6 +2339,10 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
     const int grc = try_grid_march(pl, r, ws, s);
     if (grc != kNotGrid) return grc;
   }
+  // the plan's streams and events are shared by every caller of the plan: one at a time hands
+  // them work, so that no caller's fork, join or copy takes another's event
+  std::unique_lock<std::recursive_mutex> lock(g_aux_mu, std::defer_lock);
+  if (sink) lock.lock();
   {
     const int crc = try_cluster_march(pl, r, ws, s);
     if (crc != kNotCluster) {
@@ -2360,10 +2364,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   const size_t slot = ws_layout(pl, G).total;
   const int conc = std::max(
       1, (int)std::min<size_t>({(size_t)ngroups, ws_bytes / slot, (size_t)(r->conc > 0 ? r->conc : conc_limit())}));
-  // the plan's streams and events are shared by every caller of the plan: one at a time hands
-  // them work, so that no caller's fork or join takes another's event
-  std::unique_lock<std::recursive_mutex> lock(g_aux_mu, std::defer_lock);
-  if (conc > 1 || sink) lock.lock();
+  if (conc > 1 && !lock.owns_lock()) lock.lock();
   cudaStream_t st[kMaxConcurrentGroups];
   for (int j = 0; j < conc; j++) st[j] = conc > 1 ? pl->aux[j] : s;
   if (conc > 1 || sink) BPM_CUDA_TRY(cudaEventRecord(pl->ev_fork, s));

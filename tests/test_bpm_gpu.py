@@ -695,3 +695,38 @@ def test_one_launch_scattering_sums_stay_with_their_plane(bpm, size, mode):
     for k in (0, 1):  # (nothing has scattered before plane 2: 0 / 0 in g)
         a, b = got[0][k][2:], np.asarray(want[1 + k])[2:]
         assert np.all(np.abs(a - b) <= TOL * np.abs(b)), k
+
+
+@pytest.mark.parametrize("side,batches,launch", [(64, (1, 96, 7, 32), None), (128, (1, 4, 2, 3), None),
+                                                 (128, (24, 1, 9, 2), {"cluster": 1}), (128, (1, 8, 2, 16), {"cluster": 2})])
+def test_streamed_host_output_from_several_threads(bpm, side, batches, launch):
+    """Threads whose marches of one plan stream to page-locked memory at once, by the whole-march
+    cluster kernel and by the pass kernels, with batches of different lengths: every result is the
+    one that the call gives alone, so no copy went out on another caller's event."""
+    import threading
+    import torch
+    nz = 6
+    g = torch.Generator(device="cuda").manual_seed(side)
+    dn = .02 * torch.randn((nz, side, side), device="cuda", generator=g)
+    jobs = []
+    for i, b in enumerate(batches):
+        tilt = torch.rand((b, 1, 1), device="cuda", generator=g) - .5
+        u0 = torch.exp(1j * tilt * torch.arange(side, device="cuda")[None, None, :]).to(torch.complex64)
+        u0 = u0.expand(b, side, side).contiguous()
+        want = bpm.bpm_3d_batched((side, side, nz), (.1, .1, .1), u0=u0, dn=dn, n0=1.33, launch=launch).cpu()
+        jobs.append((u0, want, torch.empty((b, nz, side, side), dtype=torch.complex64, pin_memory=True)))
+    bad = []
+
+    def work(u0, want, out):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(15):
+                out.zero_()
+                bpm.bpm_3d_batched((side, side, nz), (.1, .1, .1), u0=u0, dn=dn, n0=1.33, out=out, launch=launch)
+                if not torch.equal(out, want):
+                    bad.append(tuple(out.shape))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad, bad
