@@ -1205,8 +1205,12 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
 // of the exchange in between have arrived, which they sent after receiving the earlier ones.
 // The FFTs, pointwise helpers and the weighted sums are those of the pass kernels, so the
 // results are the same bits (at 64, where the pass kernels use the tile FFT, the same to FP32
-// rounding). Every wait is bounded in time; a block that gives up finishes the march without
-// further waits (its output is then wrong) and records it for bpm_device_status.
+// rounding). Every wait is bounded in time; a block with a thread that gave up in a step records it
+// for bpm_device_status and leaves the march after the step, so its peers give up in their turn, no
+// mbarrier receives more than a few exchanges ahead, and the planes that are left stay unwritten.
+// The threads agree on leaving by a flag per step parity, set before the step's last block barrier
+// and read in the next step, before the wait for its tiles, where it costs least (64^2 180.5 -> 181
+// us, 128^2 514 -> 518; __syncthreads_or in every sending: 186 -> 192, 523 -> 545).
 // ---------------------------------------------------------------------------------------
 __device__ int g_march_status;                                // nonzero once a wait gave up
 
@@ -1216,6 +1220,7 @@ struct ClusterArgs {
   const float2* u0;  // (batch, N, N)
   int nz;
   unsigned long long wait_ns;
+  int starve;        // -1; the wait self-test: the mbarrier told to expect 16 bytes that never come
 };
 
 template <int N>
@@ -1239,9 +1244,9 @@ struct ClusterCfg {
   static_assert(TS % 2 == 0 && T >= C, "cluster shape");
 };
 
-// Waits for a phase of an mbarrier whose arrivals come from the cluster; once a wait of the
-// thread has given up (dead), further ones return at once.
-__device__ __forceinline__ void cluster_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, bool& dead) {
+// Waits for a phase of an mbarrier whose arrivals come from the cluster; false where it gives up,
+// after which (dead) further waits of the thread return at once.
+__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, bool& dead) {
   auto ready = [&] {
     uint32_t ok;
     asm volatile(
@@ -1253,14 +1258,15 @@ __device__ __forceinline__ void cluster_wait(uint64_t* bar, uint32_t parity, uns
         : "memory");
     return ok != 0;
   };
-  if (dead || ready()) return;
+  if (dead || ready()) return true;
   const uint64_t t0 = tc::global_ns();
   while (!ready())
     if (tc::global_ns() - t0 > limit_ns) {
       dead = true;
       atomicExch(&g_march_status, 1);
-      return;
+      return false;
     }
+  return true;
 }
 
 // the address of this block's shared-memory address a in the cluster's block r
@@ -1287,6 +1293,7 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
   float2* tw = stage0 + 2 * Cfg::EX;
   float2* sums = tw + Cfg::TWPAD + S * Cfg::BUF;  // weighted: the N column sums
   __shared__ __align__(8) uint64_t bar[3];        // K, R and sums
+  __shared__ int gave_up[2];                      // a thread gave up in the step, by its parity
   const int tid = threadIdx.x, seq = tid / L, t = tid % L, lane = tid & 31;
   float2* buf = tw + Cfg::TWPAD + seq * Cfg::BUF;
   const int row = c * S + seq;        // this sequence's row, and its column
@@ -1297,6 +1304,8 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
   if (tid == 0) {
     for (int i = 0; i < 3; i++) tc::mbar_init(&bar[i], 1);
     tc::fence_mbar_init();
+    gave_up[0] = gave_up[1] = 0;
+    if (a.starve >= 0) tc::mbar_expect_bytes(&bar[a.starve], 16);
   }
   for (int k = tid; k < WarpFft<N, L>::TW; k += Cfg::T) tw[k] = p.wtw[k];
   // constants of the lane's column entries y = t + L m: the propagator table, or kx^2 and ky^2
@@ -1313,6 +1322,13 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
   const float kx2 = __ldg(q.kx2 + row);
   cl.sync();  // every block's mbarriers are initialised
 
+  auto wait = [&](uint64_t* b, uint32_t ph) {
+    if (!cluster_wait(b, ph, a.wait_ns, dead)) gave_up[ph] = 1;
+  };
+  // (an mbarrier is armed once its last phase is complete, as far as this thread's waits were met)
+  auto expect = [&](uint64_t* b, uint32_t bytes) {
+    if (tid == 0 && !dead) tc::mbar_expect_tx(b, bytes);
+  };
   // sends the sequence's values v[m] (element t + L m) to the blocks that own those elements
   auto send = [&](const float2 (&v)[E], float2* dst, float2* stage, uint64_t* b) {
 #pragma unroll
@@ -1322,7 +1338,7 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
     }
     tc::fence_proxy_async();
     __syncthreads();
-    if (tid == 0) tc::mbar_expect_tx(b, (uint32_t)(Cfg::EX * sizeof(float2)));
+    expect(b, (uint32_t)(Cfg::EX * sizeof(float2)));
     if (tid < C) {
       const int peer = (tid + c) % C;
       asm volatile(
@@ -1378,7 +1394,8 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
     float dn0 = (p.mean_mode == BPM_MEAN_SIMPLE && p.slice_dn0) ? p.slice_dn0[z] : 0.f;
 
     // ---- column phase ----
-    cluster_wait(&bar[0], ph, a.wait_ns, dead);
+    if (*(volatile int*)&gave_up[ph ^ 1]) break;  // in the step before
+    wait(&bar[0], ph);
     receive(v, K);
     warp_fft<N, false, L>(v, buf, tw, t);
     if (weighted) {
@@ -1394,13 +1411,13 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
         sm.x += __shfl_xor_sync(0xffffffffu, sm.x, o);
         sm.y += __shfl_xor_sync(0xffffffffu, sm.y, o);
       }
-      if (tid == 0) tc::mbar_expect_tx(&bar[2], (uint32_t)(N * sizeof(float2)));
+      expect(&bar[2], (uint32_t)(N * sizeof(float2)));
       for (int r = t; r < C; r += L)
         asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(
                          peer_addr(tc::smem_u32(sums + row), r)),
                      "f"(sm.x), "f"(sm.y), "r"(peer_addr(tc::smem_u32(&bar[2]), r))
                      : "memory");
-      cluster_wait(&bar[2], ph, a.wait_ns, dead);
+      wait(&bar[2], ph);
       __syncwarp();
       dn0 = weighted_total<N / 32>(N, lane, [&](int i) { return sums[i]; });
       n_eff = q.n00f + dn0;  // mult_propagator_buff, bpm_3d_kernels.cl:482
@@ -1427,7 +1444,7 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
                     ? mask_from_complex(mk[m], p.unit_k)
                     : mask_from_real(mk[m].x, p.unit_k, t + L * m, row, N, N, p.absorb, p.taper);
     }
-    cluster_wait(&bar[1], ph, a.wait_ns, dead);
+    wait(&bar[1], ph);
     receive(v, R);
     warp_fft<N, true, L>(v, buf, tw, t);
     if (p.do_mask) {
@@ -1447,12 +1464,16 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
 #pragma unroll
     for (int m = 0; m < E; m++) store_plane(z, m, u[m]);  // after the tiles are on their way
   }
-  if (dead) {  // copies that were late still land before any block of the cluster leaves
+  // No block leaves while its tiles are being read or another's are under way to it. Where all
+  // waits were met they have all landed. Where one gave up, tiles that came late may have been
+  // sent just before the sender's first barrier: they get 5 ms, sender and receiver in place.
+  cl.sync();
+  if (dead) {
     const uint64_t t0 = tc::global_ns();
     while (tc::global_ns() - t0 < 5000000ull) {
     }
   }
-  cl.sync();  // no block leaves while its tiles are being read or another may still send to it
+  cl.sync();
 }
 
 // ---------------------------------------------------------------------------------------
@@ -2201,6 +2222,12 @@ bool cluster_default(int n, int mean_mode, int batch) {
   return n == 64 || (n == 128 && (weighted || batch <= 32)) || (n == 256 && weighted && batch <= 4);
 }
 
+// the limit of a whole-march kernel's waits, and what the wait self-test withholds (-1: nothing)
+struct MarchWaits {
+  unsigned long long ns = kMarchWaitNs;
+  int starve = -1;
+};
+
 template <int N>
 struct ClusterK {
   static cudaLaunchConfig_t config(unsigned batch, cudaStream_t s, cudaLaunchAttribute* at) {
@@ -2237,7 +2264,7 @@ struct ClusterK {
       return ok;
     }) == 1;
   }
-  static int launch(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
+  static int launch(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s, const MarchWaits& w) {
     MarchCtx c = make_ctx(pl, r, ws, 0, r->batch, group_size(pl, r));
     ClusterArgs a;
     a.rp = c.rp;
@@ -2245,7 +2272,8 @@ struct ClusterK {
     a.cp = c.cp;
     a.u0 = static_cast<const float2*>(r->u0);
     a.nz = pl->d.nz;
-    a.wait_ns = kMarchWaitNs;
+    a.wait_ns = w.ns;
+    a.starve = w.starve;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = config((unsigned)r->batch, s, at);
     BPM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cluster_march_kernel<N>, a));
@@ -2256,14 +2284,14 @@ struct ClusterK {
 
 // kNotCluster when the request is not for the cluster kernel, else its launch status
 constexpr int kNotCluster = 1;
-int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
+int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s, const MarchWaits& w = {}) {
   const bpm_grid_desc& d = pl->d;
   const bool want = r->cluster == 1 || (r->cluster == 0 && cluster_default(d.nx, d.mean_mode, r->batch));
   if (d.nx != d.ny || !want || r->scatter_p || r->ckpt || !pl->wtw_x || !pl->wtw_y) return kNotCluster;
   switch (d.nx) {
-    case 64: return ClusterK<64>::ready() ? ClusterK<64>::launch(pl, r, ws, s) : kNotCluster;
-    case 128: return ClusterK<128>::ready() ? ClusterK<128>::launch(pl, r, ws, s) : kNotCluster;
-    case 256: return ClusterK<256>::ready() ? ClusterK<256>::launch(pl, r, ws, s) : kNotCluster;
+    case 64: return ClusterK<64>::ready() ? ClusterK<64>::launch(pl, r, ws, s, w) : kNotCluster;
+    case 128: return ClusterK<128>::ready() ? ClusterK<128>::launch(pl, r, ws, s, w) : kNotCluster;
+    case 256: return ClusterK<256>::ready() ? ClusterK<256>::launch(pl, r, ws, s, w) : kNotCluster;
   }
   return kNotCluster;
 }
@@ -2299,7 +2327,7 @@ bool grid_default(const bpm_grid_desc& d, int batch, cudaStream_t s) {
 }
 
 constexpr int kNotGrid = 1;
-int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s) {
+int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s, const MarchWaits& w = {}) {
   const bpm_grid_desc& d = pl->d;
   if (d.nx < 128 || d.ny < 128 || r->ckpt || r->cluster == 2 || r->group || r->conc || r->col_block || r->col_fuse ||
       !grid_default(d, r->batch, s) || ((d.nx == 1024 || d.ny == 1024) && !warp1024_enabled()))
@@ -2314,7 +2342,8 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
   a.u0 = static_cast<const float2*>(r->u0);
   a.nz = d.nz;
   a.counter = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + ws_layout(pl, G).counter);
-  a.wait_ns = kMarchWaitNs;
+  a.wait_ns = w.ns;
+  a.starve = w.starve >= 0 ? 1 : 0;
   return grid_march_launch(d.nx, d.ny, a, r->batch, s);
 }
 
@@ -2851,6 +2880,28 @@ extern "C" int bpm_propagate_to_host(bpm_plan* pl, const bpm_request* r, void* h
   }
   HostSink h{static_cast<char*>(host_out), chunk_planes};
   return enqueue_march(pl, r, ws, ws_bytes, static_cast<cudaStream_t>(stream), &h);
+}
+
+extern "C" int bpm_march_timeout_selftest(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
+                                          double wait_ms, int starve, void* stream) {
+  clear_error();
+  if (!pl) { set_error("plan is NULL"); return BPM_ERR_ARG; }
+  if (!(wait_ms > 0) || wait_ms > 1000.) { set_error("wait_ms must be in (0, 1000]"); return BPM_ERR_ARG; }
+  if (starve < 0 || starve > 2) { set_error("starve must be 0, 1 or 2"); return BPM_ERR_ARG; }
+  int rc = check_request(pl, r);
+  if (rc || (rc = check_workspace(pl, r, ws, ws_bytes))) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const MarchWaits w{(unsigned long long)(wait_ms * 1e6), starve};
+  rc = r->cluster == 1 ? try_cluster_march(pl, r, ws, s, w) : try_grid_march(pl, r, ws, s, w);
+  if (rc == kNotCluster || rc == kNotGrid) {
+    set_error("the request does not march in one launch of this kind");
+    return BPM_ERR_UNSUPPORTED;
+  }
+  if (rc) return rc;
+  BPM_CUDA_TRY(cudaStreamSynchronize(s));
+  int v = 0;
+  if ((rc = march_status(1, &v))) return rc;
+  return v ? BPM_ERR_TIMEOUT : BPM_OK;
 }
 
 extern "C" int bpm_launch_pass(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes, int pass, int z,

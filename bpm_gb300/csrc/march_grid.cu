@@ -12,7 +12,8 @@
 // the finished plane is written while the team gathers.
 //
 // The blocks of a grid wait on one another, so it is launched cooperatively (every block
-// resident at once) and every wait is bounded in time. FFTs, masks, propagator and weighted sums
+// resident at once) and every wait is bounded in time: a block that gives up one records it for
+// bpm_device_status and marches on without waiting, to a wrong result. FFTs, masks, propagator and weighted sums
 // are those of the pass kernels, so the fields are the same bits; the scattering sums are added
 // per block of C columns, not of 16, and agree to FP32 rounding.
 #include <algorithm>
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
   // plane z's behind the gathering of its row phase, when the other blocks may already be storing
   // those of plane z + 1. They store plane z + 2's only after block 0 has arrived once more.
   auto scat_part = [&](int z) { return q.scat_part + ((size_t)(2 * gl + (z & 1)) * NB) * 2; };
-  unsigned target = 0;
+  unsigned target = a.starve;
   bool dead = false;
 
   auto arrive = [&] {

@@ -15,6 +15,7 @@ struct GridMarchArgs {
   int nz;
   unsigned* counter; // kGridCounterStride unsigned per field
   unsigned long long wait_ns;
+  unsigned starve;   // 0; the wait self-test: 1, an arrival that every gathering waits for in vain
 };
 
 // fields that can march at once on the current device, 0 where the grid has no such kernel

@@ -320,8 +320,8 @@ size_t debye_workspace_bytes(const debye_desc* desc);
 /* Sticky device-side status of the kernels with bounded waits: nonzero once one of the
  * tensor-core quadrature's (an mbarrier that a TMA copy or a tensor-core product should
  * complete) or one of the whole-march kernels' (tiles or arrivals of the field's other blocks)
- * gave up after 2 s, in which case that launch left its outputs unwritten or wrong. Synchronises with the
- * device to read it; clear != 0 resets it to 0. A negative bpm_status on a CUDA error.
+ * gave up after 2 s, in which case that launch left its outputs unwritten or wrong. Synchronises
+ * with the device to read it; clear != 0 resets it to 0. A negative bpm_status on a CUDA error.
  * No counterpart in the reference (its OpenCL kernels have no such waits). */
 int bpm_device_status(int clear);
 
@@ -332,6 +332,17 @@ int bpm_device_status(int clear);
  * BPM_OK if the product completed, another negative status on a CUDA error. Allocates its
  * own small buffers and synchronises the device. No counterpart in the reference. */
 int debye_tc_timeout_selftest(double wait_ms);
+
+/* The same for the whole-march kernels: runs the request once by the cluster kernel
+ * (req->cluster 1) or as one cooperative launch (else), with waits that give up after wait_ms
+ * (0 < wait_ms <= 1000) and one that cannot be met: starve 0, 1, 2 is the cluster kernel's
+ * exchange from rows to columns, from columns to rows, or of the weighted sums (one that the
+ * march does not wait for is met); in the cooperative launch any value withholds an arrival.
+ * Returns BPM_ERR_TIMEOUT when a wait gave up (the status is cleared again; the outputs are
+ * unwritten or wrong), BPM_OK if all were met, BPM_ERR_UNSUPPORTED where the request does not
+ * march in one launch of that kind. Synchronises the stream. No counterpart in the reference. */
+int bpm_march_timeout_selftest(bpm_plan* plan, const bpm_request* req, void* workspace, size_t workspace_bytes,
+                               double wait_ms, int starve, void* stream);
 
 /* Compute the focus field on the full (nz, ny, nx) grid centred at index n/2.
  * Replaces bpm/psf/_focus_fields_debye.py:focus_field_debye (:48-146): the debye_wolf

@@ -730,3 +730,48 @@ def test_streamed_host_output_from_several_threads(bpm, side, batches, launch):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not bad, bad
+
+
+@pytest.mark.parametrize("size,mode,cluster,starve", [((64, 64, 40), "weighted", 1, 0), ((64, 64, 40), "ignore", 1, 1),
+                                                      ((128, 128, 40), "weighted", 1, 2), ((128, 128, 3), "simple", 1, 1),
+                                                      ((256, 256, 40), "weighted", 1, 1), ((256, 256, 2), "ignore", 1, 0),
+                                                      ((256, 128, 9), "weighted", 0, 0), ((512, 512, 4), "ignore", 0, 0)])
+def test_whole_march_wait_runs_out_and_reports(bpm, size, mode, cluster, starve):
+    """A bounded wait of the whole-march kernels that cannot be met (an exchange told to expect 16
+    bytes that never come, or an arrival too many) gives up after 20 ms and reports
+    BPM_ERR_TIMEOUT; a wait that the mode does not have is met. The context stays usable: the same
+    march afterwards is correct and leaves the status clear."""
+    import ctypes
+    import time
+    import torch
+    from bpm_gb300 import _native as N
+    from bpm_gb300.bpm3d import _ptr, _slice_tables, get_plan
+    Nx, Ny, Nz = size
+    B = 2 if Nx != 256 or Ny != 128 else 1
+    rng = np.random.default_rng(Nx + starve)
+    dn = (.03 * rng.standard_normal((Nz, Ny, Nx))).astype(np.float32)
+    d, u0 = torch.from_numpy(dn).cuda(), torch.ones((B, Ny, Nx), dtype=torch.complex64, device="cuda")
+    tabs = _slice_tables(d, 1.33, d.device) if mode == "simple" else (None, None)
+    plan = get_plan(size, (.1, .1, .1), .5, 1.33, 0, mode)
+    last = torch.empty_like(u0)
+    wsb = plan.workspace_bytes(B)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    req = N.Request(B, _ptr(u0), _ptr(d), N.DN_F32, 0, _ptr(tabs[0]), _ptr(tabs[1]), None, N.OUT_NONE, 0, _ptr(last))
+    req.cluster = cluster
+    L = N.lib()
+    for k in range(3):
+        t0 = time.perf_counter()
+        rc = L.bpm_march_timeout_selftest(plan.handle, ctypes.byref(req), _ptr(ws), wsb, 20., starve, None)
+        assert rc == N.BPM_ERR_TIMEOUT, (rc, N.last_error())
+        assert time.perf_counter() - t0 < 30
+        assert L.bpm_device_status(0) == 0
+    if mode != "weighted" and cluster:
+        assert L.bpm_march_timeout_selftest(plan.handle, ctypes.byref(req), _ptr(ws), wsb, 20., 2, None) == N.BPM_OK
+    assert L.bpm_march_timeout_selftest(plan.handle, ctypes.byref(req), _ptr(ws), wsb, 0., 0, None) == -1
+    assert L.bpm_march_timeout_selftest(plan.handle, ctypes.byref(req), _ptr(ws), wsb, 20., 3, None) == -1
+    launch = {"cluster": 1} if cluster else None
+    got = bpm.bpm_3d_batched(size, (.1, .1, .1), .5, u0, d, 1.33, return_full=False, mean_mode=mode, launch=launch)
+    o = bpm_ref.bpm_3d(size, (.1, .1, .1), lam=.5, n0=1.33, dn=dn, mean_mode=mode, return_full=False, precision="fp64")
+    for b in range(B):
+        assert rel_l2(got[b].cpu().numpy(), o) < TOL
+    assert L.bpm_device_status(0) == 0
