@@ -91,6 +91,7 @@ SIGNATURES = {
     "bpm_host_ptr_mapped": (c_int, [c_vp]),
     "bpm_device_status": (c_int, [c_int]),
     "debye_tc_timeout_selftest": (c_int, [c_double]),
+    "bpm_march_timeouts": (ctypes.c_uint, []),
     "bpm_march_timeout_selftest": (c_int, [c_vp, ctypes.POINTER(Request), c_vp, c_size, c_double, c_int, c_vp]),
     "debye_workspace_bytes": (c_size, [ctypes.POINTER(DebyeDesc)]),
     "debye_focus_field": (c_int, [ctypes.POINTER(DebyeDesc), c_vp, c_vp, c_vp, c_vp, c_vp, c_size, c_vp]),
@@ -144,6 +145,19 @@ def check(rc, what=""):
     if rc == BPM_ERR_OOM:
         raise MemoryError(msg)
     raise RuntimeError("bpm_gb300 error %d: %s" % (rc, msg))
+
+
+def march_timeouts():
+    """Waits of the whole-march kernels given up on the current device so far (bpm_march_timeouts)."""
+    return lib().bpm_march_timeouts()
+
+
+def check_marches(before, what):
+    """After a march has been waited for: RuntimeError if one of its device's marches has given up a
+    bounded wait since `before` (march_timeouts() ahead of the launch), whose results are wrong."""
+    if lib().bpm_march_timeouts() != before:
+        raise RuntimeError("%s: a march on this device gave up waiting for its other blocks; its results are "
+                           "invalid (bpm_device_status)" % what)
 
 
 def launch_count():

@@ -337,6 +337,7 @@ def _bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n0=1.,
         tabs = (tabs[0].expand(Nz).contiguous(), tabs[1].expand(Nz).contiguous())
     out_kind = (N.OUT_FIELD if return_field else N.OUT_INTENSITY) if return_full else N.OUT_NONE
     mask = precompute_mask(plan, dn_t, kind) if (dn_t is not None and mask_pays(1, Nx, Ny)) else None
+    before = None if as_tensor else N.march_timeouts()
     out, last, p, g = _run(plan, u0_t, dn_t, kind, 0, out_kind, True, return_scattering, return_g,
                            scattering_plane_ind, tabs, mask=mask)
     conv = (lambda t: t) if as_tensor else _d2h
@@ -351,6 +352,8 @@ def _bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n0=1.,
     if return_last_plane:
         lp = conv(last[0])
         result = result + (lp,) if isinstance(result, tuple) else (result, lp)
+    if not as_tensor:
+        N.check_marches(before, "bpm_3d")
     return result
 
 
@@ -468,6 +471,7 @@ def bpm_3d_batched(size, units, lam=.5, u0=None, dn=None, n0=1., return_full=Tru
         tabs = (None, None)
     out_kind = (N.OUT_FIELD if return_field else N.OUT_INTENSITY) if return_full else N.OUT_NONE
     mask = precompute_mask(plan, dn_t, kind) if (dn_t is not None and bstride == 0 and mask_pays(B, Nx, Ny)) else None
+    before = None if as_tensor and out is None else N.march_timeouts()
     if out is not None and return_full:
         host = torch.from_numpy(out) if isinstance(out, np.ndarray) else out
         vdt = torch.complex64 if return_field else torch.float32
@@ -477,6 +481,7 @@ def bpm_3d_batched(size, units, lam=.5, u0=None, dn=None, n0=1., return_full=Tru
             _run_streamed_to_host(plan, u0_t, dn_t, kind, bstride, out_kind, tabs, group, mask, host, launch=launch)
         else:
             _run_to_host(plan, u0_t, dn_t, kind, bstride, out_kind, tabs, group, mask, host, launch=launch)
+        N.check_marches(before, "bpm_3d_batched")
         return out
     vol, last, _, _ = _run(plan, u0_t, dn_t, kind, bstride, out_kind, True, slice_tabs=tabs, group=group,
                            mask=mask, launch=launch)
@@ -487,8 +492,13 @@ def bpm_3d_batched(size, units, lam=.5, u0=None, dn=None, n0=1., return_full=Tru
             raise ValueError("out must have shape %s and dtype %s" % (tuple(res.shape), res.dtype))
         host.copy_(res, non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        N.check_marches(before, "bpm_3d_batched")
         return out
-    return res if as_tensor else _d2h(res)
+    if as_tensor:
+        return res
+    res = _d2h(res)
+    N.check_marches(before, "bpm_3d_batched")
+    return res
 
 
 def _run_streamed_to_host(plan, u0_t, dn_t, kind, bstride, out_kind, tabs, group, mask, host, chunk_planes=16,
@@ -789,9 +799,14 @@ class _Bpm3d_GB300:
                 else _h2d(u0, torch.complex64, dev).reshape(1, Ny, Nx))
         kind = N.DN_NONE if self._dn_t is None else (N.DN_C64 if self._is_complex_dn else N.DN_F32)
         ok = (N.OUT_INTENSITY if return_intensity else N.OUT_FIELD) if return_full else N.OUT_NONE
+        before = None if as_tensor else N.march_timeouts()
         out, last, _, _ = _run(self._plan(absorbing_width), u0_t, self._dn_t, kind, 0, ok, True)
-        conv = (lambda t: t) if as_tensor else _d2h
-        return conv(out[0]) if return_full else conv(last[0])
+        res = out[0] if return_full else last[0]
+        if as_tensor:
+            return res
+        res = _d2h(res)
+        N.check_marches(before, "propagate")
+        return res
 
     def propagate(self, u0=None, return_full=True, return_intensity=False, absorbing_width=0, **kwargs):
         """Alias of _propagate_single."""
@@ -807,9 +822,14 @@ class _Bpm3d_GB300:
             u0_t = u0_t.reshape(1, Ny, Nx)
         kind = N.DN_NONE if self._dn_t is None else (N.DN_C64 if self._is_complex_dn else N.DN_F32)
         ok = (N.OUT_INTENSITY if return_intensity else N.OUT_FIELD) if return_full else N.OUT_NONE
+        before = None if as_tensor else N.march_timeouts()
         out, last, _, _ = _run(self._plan(absorbing_width), u0_t, self._dn_t, kind, 0, ok, True, group=group)
-        conv = (lambda t: t) if as_tensor else _d2h
-        return conv(out) if return_full else conv(last)
+        res = out if return_full else last
+        if as_tensor:
+            return res
+        res = _d2h(res)
+        N.check_marches(before, "propagate_batched")
+        return res
 
     def __repr__(self):
         return "Bpm3d class with size %s and units %s" % (self.size, self.units)

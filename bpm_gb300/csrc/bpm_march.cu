@@ -78,6 +78,7 @@ struct bpm_plan {
   cudaStream_t copy;
   cudaEvent_t ev_ready[kMaxConcurrentGroups], ev_copied;
   int max_pitch;
+  int* timeouts;    // march_timeout_words of the plan's device
   // false for a plan made by bpm_plan_derive: the device tables belong to its base plan
   bool owns_tables;
 };
@@ -1212,7 +1213,8 @@ __global__ void __launch_bounds__(FusedCfg<N>::T, 1) col_fused_kernel(ColParams 
 // and read in the next step, before the wait for its tiles, where it costs least (64^2 180.5 -> 181
 // us, 128^2 514 -> 518; __syncthreads_or in every sending: 186 -> 192, 523 -> 545).
 // ---------------------------------------------------------------------------------------
-__device__ int g_march_status;                                // nonzero once a wait gave up
+__device__ int g_march_status;    // nonzero once a wait gave up (bpm_device_status)
+__device__ int g_march_timeouts;  // waits that gave up so far (bpm_march_timeouts)
 
 struct ClusterArgs {
   RowParams rp;
@@ -1220,6 +1222,7 @@ struct ClusterArgs {
   const float2* u0;  // (batch, N, N)
   int nz;
   unsigned long long wait_ns;
+  int* timeouts;     // the kernel's word of march_timeout_words
   int starve;        // -1; the wait self-test: the mbarrier told to expect 16 bytes that never come
 };
 
@@ -1246,7 +1249,8 @@ struct ClusterCfg {
 
 // Waits for a phase of an mbarrier whose arrivals come from the cluster; false where it gives up,
 // after which (dead) further waits of the thread return at once.
-__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, bool& dead) {
+__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, int* timeouts,
+                                             bool& dead) {
   auto ready = [&] {
     uint32_t ok;
     asm volatile(
@@ -1263,7 +1267,7 @@ __device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, uns
   while (!ready())
     if (tc::global_ns() - t0 > limit_ns) {
       dead = true;
-      atomicExch(&g_march_status, 1);
+      march_gave_up(&g_march_status, &g_march_timeouts, timeouts);
       return false;
     }
   return true;
@@ -1323,7 +1327,7 @@ __global__ void __launch_bounds__(ClusterCfg<N>::T) cluster_march_kernel(Cluster
   cl.sync();  // every block's mbarriers are initialised
 
   auto wait = [&](uint64_t* b, uint32_t ph) {
-    if (!cluster_wait(b, ph, a.wait_ns, dead)) gave_up[ph] = 1;
+    if (!cluster_wait(b, ph, a.wait_ns, a.timeouts, dead)) gave_up[ph] = 1;
   };
   // (an mbarrier is armed once its last phase is complete, as far as this thread's waits were met)
   auto expect = [&](uint64_t* b, uint32_t bytes) {
@@ -2273,6 +2277,7 @@ struct ClusterK {
     a.u0 = static_cast<const float2*>(r->u0);
     a.nz = pl->d.nz;
     a.wait_ns = w.ns;
+    a.timeouts = pl->timeouts;
     a.starve = w.starve;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = config((unsigned)r->batch, s, at);
@@ -2343,6 +2348,7 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
   a.nz = d.nz;
   a.counter = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + ws_layout(pl, G).counter);
   a.wait_ns = w.ns;
+  a.timeouts = pl->timeouts ? pl->timeouts + 1 : nullptr;
   a.starve = w.starve >= 0 ? 1 : 0;
   return grid_march_launch(d.nx, d.ny, a, r->batch, s);
 }
@@ -2663,6 +2669,11 @@ int bpmgb::march_status(int clear, int* v) {
 // ---------------------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------------------
+extern "C" unsigned bpm_march_timeouts(void) {
+  volatile int* w = march_timeout_words();
+  return w ? (unsigned)w[0] + (unsigned)w[1] : 0u;
+}
+
 extern "C" int bpm_grid_check(const bpm_grid_desc* d) {
   clear_error();
   if (!d) { set_error("grid description is NULL"); return BPM_ERR_ARG; }
@@ -2716,6 +2727,7 @@ extern "C" int bpm_plan_create(const bpm_grid_desc* d, bpm_plan** out) {
   pl->n0f = (float)d->n0;
   pl->unit_k = (float)(pl->k0 * d->dz);
   cudaGetDevice(&pl->device);
+  pl->timeouts = march_timeout_words();
 
   std::vector<float2> twx(nx), twy(ny);
   for (int k = 0; k < nx; k++) {

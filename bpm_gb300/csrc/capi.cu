@@ -1,4 +1,5 @@
 // Library-wide C ABI helpers: version, thread-local error text, launch accounting.
+#include <mutex>
 #include <string>
 
 #include "common.cuh"
@@ -16,6 +17,27 @@ int cuda_fail(cudaError_t e, const char* what) {
   // leave no sticky error behind for the caller's next runtime call
   cudaGetLastError();
   return e == cudaErrorMemoryAllocation ? BPM_ERR_OOM : BPM_ERR_CUDA;
+}
+
+int* march_timeout_words() {
+  static std::mutex mu;
+  static int* words[PerDevice::kMax] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= PerDevice::kMax) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  if (!words[dev]) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 2 * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    words[dev] = static_cast<int*>(p);
+    words[dev][0] = words[dev][1] = 0;
+  }
+  return words[dev];
 }
 
 }  // namespace bpmgb

@@ -23,6 +23,12 @@ int cuda_fail(cudaError_t e, const char* what);
 // current device and cleared on request; BPM_OK or a negative status
 int march_status(int clear, int* v);
 
+// Two words in page-locked host memory for the current device (a kernel's own each): how many
+// waits of the marches on it have given up so far, which the host reads without asking the device.
+// Made on the device's first call (not under capture: bpm_plan_create makes it), kept for the
+// process; NULL if it cannot be had.
+int* march_timeout_words();
+
 // number of kernels launched by this library (bpm_launch_count)
 extern std::atomic<unsigned long long> g_launches;
 inline void count_launch(unsigned long long n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }

@@ -289,4 +289,11 @@ __device__ __forceinline__ void propagate_rows(const ColParams& p, float2 (&v)[N
 // every wait of a march kernel on other blocks gives up after 2 s
 constexpr unsigned long long kMarchWaitNs = 2000000000ull;
 
+// records that one did: the sticky device status, and the count of them in the host's word
+__device__ __forceinline__ void march_gave_up(int* status, int* count, int* host_word) {
+  atomicExch(status, 1);
+  const int n = atomicAdd(count, 1) + 1;
+  if (host_word) asm volatile("st.relaxed.sys.global.s32 [%0], %1;" ::"l"(host_word), "r"(n) : "memory");
+}
+
 }  // namespace bpmgb

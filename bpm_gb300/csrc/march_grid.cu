@@ -27,7 +27,8 @@ using namespace bpmgb;
 
 namespace {
 
-__device__ int g_grid_status;  // nonzero once a wait gave up (bpm_device_status)
+__device__ int g_grid_status;    // nonzero once a wait gave up (bpm_device_status)
+__device__ int g_grid_timeouts;  // waits that gave up so far (bpm_march_timeouts)
 
 template <int NX, int NY>
 struct GridCfg {
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(GridCfg<NX, NY>::T) grid_march_kernel(GridMarc
         if ((int)(v - target) >= 0) break;
         if (n % 64 == 0 && tc::global_ns() - t0 > a.wait_ns) {
           dead = true;
-          atomicExch(&g_grid_status, 1);
+          march_gave_up(&g_grid_status, &g_grid_timeouts, a.timeouts);
           break;
         }
       }

@@ -15,6 +15,7 @@ struct GridMarchArgs {
   int nz;
   unsigned* counter; // kGridCounterStride unsigned per field
   unsigned long long wait_ns;
+  int* timeouts;     // the kernel's word of march_timeout_words
   unsigned starve;   // 0; the wait self-test: 1, an arrival that every gathering waits for in vain
 };
 

@@ -141,6 +141,7 @@ class _Launch:
     footprint: int
     keep: list = field(default_factory=list)
     results: list = field(default_factory=list)
+    timeouts: int = 0  # N.march_timeouts() ahead of the launch
 
 
 class Server:
@@ -243,7 +244,15 @@ class Server:
         for la in self._inflight:
             if la.done.query():
                 t = time.perf_counter()
+                try:
+                    N.check_marches(la.timeouts, "bpm_3d")
+                    failed = None
+                except RuntimeError as e:
+                    failed = e
                 for en, res in zip(la.entries, la.results):
+                    if failed is not None and isinstance(en.req, BpmRequest):
+                        en.fut.set_exception(failed)
+                        continue
                     self.latencies.append(t - en.t_submit)
                     self.completed += 1
                     self.voxel_updates += en.req.voxel_updates()
@@ -292,6 +301,7 @@ class Server:
         stream = self._free_streams.pop()
         fp = sum(en.req.footprint() for en in group)
         la = _Launch(group, stream, torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), fp)
+        la.timeouts = N.march_timeouts()
         try:
             with torch.cuda.stream(stream):
                 la.start.record(stream)

@@ -325,6 +325,13 @@ size_t debye_workspace_bytes(const debye_desc* desc);
  * No counterpart in the reference (its OpenCL kernels have no such waits). */
 int bpm_device_status(int clear);
 
+/* How many waits of the whole-march kernels have given up on the current device since the library
+ * was loaded (0 before its first plan there). Read from host memory that the kernels write: it asks
+ * nothing of the device, so it is valid for launches that the caller has waited for. A caller that
+ * reads it before a march and again after waiting for its results knows from an unchanged count
+ * that they are whole. No counterpart in the reference. */
+unsigned bpm_march_timeouts(void);
+
 /* Self-test of those bounded waits: runs the tensor-core quadrature kernel once on a small
  * product whose loads announce more bytes than they deliver, so its waits give up after
  * wait_ms (0 < wait_ms <= 1000) and it leaves with the status set and its tensor memory

@@ -732,6 +732,84 @@ def test_streamed_host_output_from_several_threads(bpm, side, batches, launch):
     assert not bad, bad
 
 
+def _give_up(bpm):
+    """One march whose waits run out after 5 ms (bpm_march_timeout_selftest)."""
+    import ctypes
+    import torch
+    from bpm_gb300 import _native as N
+    from bpm_gb300.bpm3d import _ptr, get_plan
+    plan = get_plan((64, 64, 3), (.1, .1, .1), .5, 1., 0, "ignore")
+    u0 = torch.ones((1, 64, 64), dtype=torch.complex64, device="cuda")
+    wsb = plan.workspace_bytes(1)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    req = N.Request(1, _ptr(u0), None, N.DN_NONE, 0, None, None, None, N.OUT_NONE, 0, _ptr(torch.empty_like(u0)))
+    req.cluster = 1
+    torch.cuda.synchronize()
+    assert N.lib().bpm_march_timeout_selftest(plan.handle, ctypes.byref(req), _ptr(ws), wsb, 5., 0, None) == -5
+
+
+@pytest.mark.parametrize("call", ["single", "split", "batched", "batched out", "batched pinned", "batched last out",
+                                  "class", "class batched"])
+def test_a_march_that_gave_up_is_reported(bpm, monkeypatch, call):
+    """Where a call waits for its results it raises if a march gave up a bounded wait since its
+    launch, and the call after it is fine again; a device-resident result is returned as it is."""
+    import torch
+    from bpm_gb300 import bpm3d as M
+    size, units = (64, 64, 6), (.1, .1, .1)
+    u0 = np.ones((2, 64, 64), np.complex64)
+    obj = bpm.Bpm3d(size, units)
+    out = torch.empty((2, 6, 64, 64), dtype=torch.complex64, pin_memory=call == "batched pinned")
+    last = np.empty((2, 64, 64), np.complex64)
+    calls = {"single": lambda: bpm.bpm_3d(size, units, u0=u0[0]),
+             "split": lambda: bpm.bpm_3d(size, units, u0=u0[0], n_volumes=2),
+             "batched": lambda: bpm.bpm_3d_batched(size, units, u0=u0),
+             "batched out": lambda: bpm.bpm_3d_batched(size, units, u0=u0, out=out),
+             "batched pinned": lambda: bpm.bpm_3d_batched(size, units, u0=u0, out=out),
+             "batched last out": lambda: bpm.bpm_3d_batched(size, units, u0=u0, return_full=False, out=last),
+             "class": lambda: obj.propagate(u0[0]), "class batched": lambda: obj.propagate_batched(u0)}
+    want = torch.as_tensor(calls[call]()).clone()
+    L = bpm._native.lib()
+    n0 = L.bpm_march_timeouts()
+    for name in ("_run", "_run_to_host", "_run_streamed_to_host"):
+        f = getattr(M, name)
+
+        def late(*a, f=f, **kw):
+            r = f(*a, **kw)
+            _give_up(bpm)
+            return r
+        monkeypatch.setattr(M, name, late)
+    with pytest.raises(RuntimeError, match="gave up"):
+        calls[call]()
+    assert L.bpm_march_timeouts() > n0
+    dev = bpm.bpm_3d(size, units, u0=torch.from_numpy(u0[0]).cuda())
+    assert dev.is_cuda
+    monkeypatch.undo()
+    assert torch.equal(torch.as_tensor(calls[call]()), want)
+    assert L.bpm_device_status(0) == 0
+
+
+def test_server_reports_a_march_that_gave_up(bpm, monkeypatch):
+    """The requests of a launch during which a march gave up fail; the ones after it do not."""
+    from bpm_gb300.serve import BpmRequest, Server
+    req = BpmRequest((64, 64, 6), (.1, .1, .1), host=True)
+    srv = Server(max_inflight=2)
+    try:
+        want = srv.submit(req).result(60)
+        f = srv._run_bpm
+
+        def late(*a):
+            r = f(*a)
+            _give_up(bpm)
+            return r
+        monkeypatch.setattr(srv, "_run_bpm", late)
+        with pytest.raises(RuntimeError, match="gave up"):
+            srv.submit(req).result(60)
+        monkeypatch.undo()
+        assert np.array_equal(srv.submit(req).result(60), want)
+    finally:
+        srv.close()
+
+
 @pytest.mark.parametrize("size,mode,cluster,starve", [((64, 64, 40), "weighted", 1, 0), ((64, 64, 40), "ignore", 1, 1),
                                                       ((128, 128, 40), "weighted", 1, 2), ((128, 128, 3), "simple", 1, 1),
                                                       ((256, 256, 40), "weighted", 1, 1), ((256, 256, 2), "ignore", 1, 0),
