@@ -259,8 +259,9 @@ mask_precompute_kernel(const void* __restrict__ dn, int dtype, float unit_k, int
 // Means of the slices of a float32 volume (mean_mode "simple"): a cluster of 8 blocks per slice.
 // Every thread adds its values into a float pair (the exact error of each addition kept in the
 // second float), the pairs are added in FP64 in a fixed order, so a mean is the FP64 one to about
-// 2^-45 without running the volume through the FP64 pipe (1/64 of the FP32 rate). Bound by reading
-// the volume; torch's mean in FP64 wrote and read it again as doubles, and the tables went
+// 2^-45 without running the volume through the FP64 pipe (1/64 of the FP32 rate). A thread whose
+// float sums leave the FP32 range, or that meets an infinity or a NaN, adds its values again in
+// FP64. Bound by reading the volume; torch's mean in FP64 wrote and read it again as doubles, and the tables went
 // through the host.
 constexpr int kMeanThreads = 256, kMeanBlocks = 8;
 
@@ -278,8 +279,9 @@ slice_means_kernel(const float* __restrict__ dn, size_t plane, double n0, float*
   __shared__ double block_sum;
   const int z = blockIdx.y, rank = (int)cl.block_rank(), tid = threadIdx.x;
   const float* src = dn + (size_t)z * plane;
+  const bool vec = ((uintptr_t)src & 15) == 0 && plane % 4 == 0;
   float2 a[4] = {};
-  if (((uintptr_t)src & 15) == 0 && plane % 4 == 0) {
+  if (vec) {
     const float4* s4 = reinterpret_cast<const float4*>(src);
 #pragma unroll 4
     for (size_t i = (size_t)rank * kMeanThreads + tid; i < plane / 4; i += kMeanBlocks * kMeanThreads) {
@@ -294,9 +296,18 @@ slice_means_kernel(const float* __restrict__ dn, size_t plane, double n0, float*
       pair_add(a[0], __ldg(src + i));
   }
   double s = 0.;
+  bool finite = true;
 #pragma unroll
-  for (int k = 0; k < 4; k++)  // an infinite sum has no error term
-    s += isinf(a[k].x) ? (double)a[k].x : (double)a[k].x + (double)a[k].y;
+  for (int k = 0; k < 4; k++) {
+    s += (double)a[k].x + (double)a[k].y;
+    finite = finite && isfinite(a[k].x);
+  }
+  if (!finite) {
+    s = 0.;
+    const int w = vec ? 4 : 1;
+    for (size_t i = (size_t)rank * kMeanThreads + tid; i < plane / w; i += kMeanBlocks * kMeanThreads)
+      for (int k = 0; k < w; k++) s += (double)__ldg(src + w * i + k);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((tid & 31) == 0) warp_sum[tid >> 5] = s;

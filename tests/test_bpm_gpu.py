@@ -853,3 +853,29 @@ def test_whole_march_wait_runs_out_and_reports(bpm, size, mode, cluster, starve)
     for b in range(B):
         assert rel_l2(got[b].cpu().numpy(), o) < TOL
     assert L.bpm_device_status(0) == 0
+
+
+@pytest.mark.parametrize("shape,offset", [((4, 16, 16), 0), ((4, 64, 48), 1), ((4, 1024, 512), 0)])
+def test_slice_means_beyond_float32_sums(bpm, shape, offset):
+    """Slices whose float32 sums overflow while the FP64 ones do not, and slices with infinities
+    and NaN: the tables are numpy's FP64 means rounded once (the redone sums are FP64 sums, so
+    they differ from numpy's in the last bits of FP64 only)."""
+    import torch
+    from bpm_gb300.bpm3d import _slice_tables
+    rng = np.random.default_rng(shape[1])
+    a = (rng.uniform(-1, 1, shape) * 1e-2).astype(np.float32)
+    a[0] = 3e38 * rng.choice([1, 1, -.5], shape[1:])
+    a[1, 0, :4] = np.inf, 1., 2., 3.
+    a[2, -1, -3:] = np.inf, 0., -np.inf
+    a[3, 2, 5] = np.nan
+    buf = torch.zeros(a.size + offset, device="cuda")
+    dn = buf[offset:].reshape(shape)
+    dn.copy_(torch.from_numpy(a))
+    sn, sd = _slice_tables(dn, 1.33, buf.device)
+    with np.errstate(invalid="ignore"):
+        m = a.astype(np.float64).mean(axis=(1, 2))
+    assert np.isfinite(m[0]) and m[1] == np.inf and np.isnan(m[2]) and np.isnan(m[3])
+    for got, want in ((sn, 1.33 + m), (sd, m)):
+        got = got.cpu().numpy()
+        assert np.array_equal(got[1:], want[1:].astype(np.float32), equal_nan=True)
+        assert abs(got[0] - want[0]) <= 2.**-23 * abs(want[0])
