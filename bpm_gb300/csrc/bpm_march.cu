@@ -2221,9 +2221,17 @@ int sink_copy(bpm_plan* pl, const bpm_request* r, const HostSink& h, int b0, int
 //   256^2: the weighted mode up to 4 fields (8.8 against 9.6 for 1 field and 11.0 for 4); a field
 //     fills 16 SMs there, so 8 fields take 17.6 against 12.4, and without the sums one field
 //     6.7 against 4.8.
+// With a host sink (sink_bytes: of a plane of all fields, 0 without one) the volume is copied after
+// the cluster march and during the march of the pass kernels, so what it gains per step has to be
+// more than the copy of a plane takes, about 5 us per MB (GB300, ms for the whole call, cluster kernel
+// against passes): 64^2 as without (64 fields of complex output, 2 MB, 1.05 against 1.21); 128^2 weighted
+// 12 fields of intensities (768 KB) 1.27 against 1.39, 16 1.67 against 1.46, 4 of complex output (512 KB)
+// 0.93 against 1.23, 8 1.42 against 1.35; 128^2 otherwise 4 fields of intensities (256 KB) 0.61 against
+// 0.73, 8 0.94 against 0.89, 2 of complex output (256 KB) 0.62 against 0.71, 4 0.79 against 0.75; 256^2
+// weighted 1 field of intensities (256 KB) 1.35 against 1.45, 1 of complex output 1.54 against 1.46.
 // BPM_GB300_CLUSTER=1 takes it wherever it serves, =0 nowhere, and a side length (64, 128 or
 // 256) wherever it serves up to that side.
-bool cluster_default(int n, int mean_mode, int batch) {
+bool cluster_default(int n, int mean_mode, int batch, size_t sink_bytes) {
   static const int max_side = [] {
     const char* e = getenv("BPM_GB300_CLUSTER");
     if (!e) return -1;
@@ -2234,6 +2242,7 @@ bool cluster_default(int n, int mean_mode, int batch) {
   }();
   if (max_side >= 0) return n <= max_side;
   const bool weighted = mean_mode == BPM_MEAN_WEIGHTED;
+  if (n != 64 && sink_bytes > (n == 128 && weighted ? 768u << 10 : 256u << 10)) return false;
   return n == 64 || (n == 128 && (weighted || batch <= 32)) || (n == 256 && weighted && batch <= 4);
 }
 
@@ -2300,9 +2309,11 @@ struct ClusterK {
 
 // kNotCluster when the request is not for the cluster kernel, else its launch status
 constexpr int kNotCluster = 1;
-int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s, const MarchWaits& w = {}) {
+int try_cluster_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStream_t s, bool sink,
+                      const MarchWaits& w = {}) {
   const bpm_grid_desc& d = pl->d;
-  const bool want = r->cluster == 1 || (r->cluster == 0 && cluster_default(d.nx, d.mean_mode, r->batch));
+  const size_t sink_bytes = sink ? (size_t)r->batch * d.nx * d.ny * (r->out_kind == BPM_OUT_FIELD ? 8 : 4) : 0;
+  const bool want = r->cluster == 1 || (r->cluster == 0 && cluster_default(d.nx, d.mean_mode, r->batch, sink_bytes));
   if (d.nx != d.ny || !want || r->scatter_p || r->ckpt || !pl->wtw_x || !pl->wtw_y) return kNotCluster;
   switch (d.nx) {
     case 64: return ClusterK<64>::ready() ? ClusterK<64>::launch(pl, r, ws, s, w) : kNotCluster;
@@ -2390,7 +2401,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   std::unique_lock<std::recursive_mutex> lock(g_aux_mu, std::defer_lock);
   if (sink) lock.lock();
   {
-    const int crc = try_cluster_march(pl, r, ws, s);
+    const int crc = try_cluster_march(pl, r, ws, s, sink != nullptr);
     if (crc != kNotCluster) {
       if (crc != BPM_OK) return crc;
       if (sink) {
@@ -2915,7 +2926,7 @@ extern "C" int bpm_march_timeout_selftest(bpm_plan* pl, const bpm_request* r, vo
   if (rc || (rc = check_workspace(pl, r, ws, ws_bytes))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const MarchWaits w{(unsigned long long)(wait_ms * 1e6), starve};
-  rc = r->cluster == 1 ? try_cluster_march(pl, r, ws, s, w) : try_grid_march(pl, r, ws, s, w);
+  rc = r->cluster == 1 ? try_cluster_march(pl, r, ws, s, false, w) : try_grid_march(pl, r, ws, s, w);
   if (rc == kNotCluster || rc == kNotGrid) {
     set_error("the request does not march in one launch of this kind");
     return BPM_ERR_UNSUPPORTED;

@@ -114,7 +114,9 @@ typedef struct {
                                     Default: the cluster kernel at 64, at 128 but for large
                                     batches without the weighted sums, and for 3 or 4 weighted
                                     fields of 256; one cooperative launch for one or a few
-                                    fields of other grids from 128 up; else pass kernels        */
+                                    fields of other grids from 128 up; else pass kernels. Into a
+                                    host sink (bpm_propagate_to_host) from 128 up only the
+                                    cluster kernel, where a plane of all fields is small        */
   int col_fuse;                  /* weighted mode: 1 = one column pass per step (forward FFT,
                                     plane-wide sums across a thread-block cluster of the field's
                                     blocks, propagator, inverse FFT) where ny <= 512, nx <= 512
