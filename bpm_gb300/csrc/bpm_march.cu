@@ -70,6 +70,8 @@ struct bpm_plan {
   float* gw;        // g-factor weights cos(theta)^2
   float k0f, dzf, n0f, unit_k;
   double k0;
+  // held by the caller that is handing work to the streams below
+  std::recursive_mutex* mu;
   // streams on which groups of fields march concurrently, with their fork/join events
   cudaStream_t aux[kMaxConcurrentGroups];
   cudaEvent_t ev_fork, ev_join[kMaxConcurrentGroups];
@@ -2375,8 +2377,6 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
   return grid_march_launch(d.nx, d.ny, a, r->batch, s);
 }
 
-std::recursive_mutex g_aux_mu;
-
 // All groups of a request. With room for several workspace slots, groups march
 // concurrently on the plan's auxiliary streams (forked from and joined back to s through
 // events, which also captures into a CUDA graph as parallel branches), so one group's
@@ -2398,7 +2398,7 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   }
   // the plan's streams and events are shared by every caller of the plan: one at a time hands
   // them work, so that no caller's fork, join or copy takes another's event
-  std::unique_lock<std::recursive_mutex> lock(g_aux_mu, std::defer_lock);
+  std::unique_lock<std::recursive_mutex> lock(*pl->mu, std::defer_lock);
   if (sink) lock.lock();
   {
     const int crc = try_cluster_march(pl, r, ws, s, sink != nullptr);
@@ -2720,9 +2720,10 @@ extern "C" int bpm_grid_check(const bpm_grid_desc* d) {
   return BPM_OK;
 }
 
-// the plan's own streams and events (no device synchronisation)
+// the plan's own streams and events (no device synchronisation) and their lock
 static cudaError_t create_plan_streams(bpm_plan* pl) {
   cudaError_t e;
+  pl->mu = new std::recursive_mutex();
   for (int i = 0; i < kMaxConcurrentGroups; i++) {
     if ((e = cudaStreamCreateWithFlags(&pl->aux[i], cudaStreamNonBlocking))) return e;
     if ((e = cudaEventCreateWithFlags(&pl->ev_join[i], cudaEventDisableTiming))) return e;
@@ -2831,6 +2832,7 @@ extern "C" int bpm_plan_derive(const bpm_plan* base, int nz, bpm_plan** out) {
   for (int i = 0; i < kMaxConcurrentGroups; i++) pl->aux[i] = nullptr, pl->ev_join[i] = pl->ev_ready[i] = nullptr;
   pl->ev_fork = pl->ev_copied = nullptr;
   pl->copy = nullptr;
+  pl->mu = nullptr;
   cudaError_t e = create_plan_streams(pl);
   if (e) {
     bpm_plan_destroy(pl);
@@ -2863,6 +2865,7 @@ extern "C" int bpm_plan_destroy(bpm_plan* pl) {
   if (pl->ev_fork) cudaEventDestroy(pl->ev_fork);
   if (pl->copy) cudaStreamDestroy(pl->copy);
   if (pl->ev_copied) cudaEventDestroy(pl->ev_copied);
+  delete pl->mu;
   delete pl;
   return BPM_OK;
 }
@@ -3025,7 +3028,7 @@ extern "C" int bpm_exec_create(bpm_plan* pl, const bpm_request* r, void* ws, siz
   if (!pl || !out) { set_error("plan/out is NULL"); return BPM_ERR_ARG; }
   int rc = check_request(pl, r);
   if (rc) return rc;
-  std::lock_guard<std::recursive_mutex> lock(g_aux_mu);  // the plan's streams join the capture
+  std::lock_guard<std::recursive_mutex> lock(*pl->mu);  // the plan's streams join the capture
   cudaStream_t s;
   BPM_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   unsigned long long before = g_launches.load();

@@ -901,3 +901,43 @@ def test_host_output_streams_beside_the_march(bpm, side, mode, field, batch, str
     assert (bpm.launch_count() - n0 >= 2 * (nz - 1)) == streams
     # (at 64 the pass kernels' tile FFT rounds differently; the same kernel marched there)
     assert torch.equal(out, want.cpu())
+
+
+def test_plans_take_their_own_lock(bpm):
+    """A thread that hands a long march in concurrent groups to the device does not keep another
+    thread's short march, of another plan, from being handed over: its calls take a fraction of
+    the long one's (they waited for the whole of it when all plans shared a lock)."""
+    import threading
+    import time
+    import torch
+    kw = dict(units=(.1, .1, .1), lam=.5, n0=1.33, batch=4, use_graph=False, group=2, launch={"cluster": 2})
+    long, short = bpm.BatchedMarch((32, 32, 200), **kw), bpm.BatchedMarch((32, 32, 2), **kw)
+    assert long.plan is not short.plan
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    stop, spent = threading.Event(), []
+    for m, s in ((long, s1), (short, s2)):
+        m.run(s.cuda_stream)
+    torch.cuda.synchronize()
+
+    def work():
+        while not stop.is_set():
+            t = time.perf_counter()
+            long.run(s1.cuda_stream)
+            spent.append(time.perf_counter() - t)
+            s1.synchronize()
+
+    th = threading.Thread(target=work)
+    th.start()
+    try:
+        while len(spent) < 5:
+            time.sleep(.001)
+        took = []
+        for _ in range(300):
+            t = time.perf_counter()
+            short.run(s2.cuda_stream)
+            took.append(time.perf_counter() - t)
+            s2.synchronize()
+    finally:
+        stop.set()
+        th.join()
+    assert np.percentile(took, 80) < .25 * np.median(spent), (np.percentile(took, [50, 80, 95]), np.median(spent))
