@@ -2377,11 +2377,23 @@ int try_grid_march(const bpm_plan* pl, const bpm_request* r, void* ws, cudaStrea
   return grid_march_launch(d.nx, d.ny, a, r->batch, s);
 }
 
+// whether stream a is part of a capture that s is not: work from s may not be ordered before a's
+bool in_another_capture(cudaStream_t a, cudaStream_t s) {
+  cudaStreamCaptureStatus sa = cudaStreamCaptureStatusNone, ss = cudaStreamCaptureStatusNone;
+  unsigned long long ia = 0, is = 0;
+  if (cudaStreamGetCaptureInfo(a, &sa, &ia) != cudaSuccess || cudaStreamGetCaptureInfo(s, &ss, &is) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return sa != cudaStreamCaptureStatusNone && (ss == cudaStreamCaptureStatusNone || ia != is);
+}
+
 // All groups of a request. With room for several workspace slots, groups march
 // concurrently on the plan's auxiliary streams (forked from and joined back to s through
 // events, which also captures into a CUDA graph as parallel branches), so one group's
 // kernels fill the device while another's run their tail waves; otherwise they march one
-// after the other on s. Groups marching at the same time are enqueued step by step in
+// after the other on s, also while the plan's streams are part of another caller's capture (from
+// its march to the capture's end). Groups marching at the same time are enqueued step by step in
 // turn, so work (and, with a host sink, the finished planes handed to the copy stream)
 // reaches the device in the order it can run.
 int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes, cudaStream_t s,
@@ -2419,9 +2431,10 @@ int enqueue_march(bpm_plan* pl, const bpm_request* r, void* ws, size_t ws_bytes,
   const int G = group_size(pl, r);
   const int ngroups = (r->batch + G - 1) / G;
   const size_t slot = ws_layout(pl, G).total;
-  const int conc = std::max(
+  int conc = std::max(
       1, (int)std::min<size_t>({(size_t)ngroups, ws_bytes / slot, (size_t)(r->conc > 0 ? r->conc : conc_limit())}));
   if (conc > 1 && !lock.owns_lock()) lock.lock();
+  if (conc > 1 && in_another_capture(pl->aux[0], s)) conc = 1;
   cudaStream_t st[kMaxConcurrentGroups];
   for (int j = 0; j < conc; j++) st[j] = conc > 1 ? pl->aux[j] : s;
   if (conc > 1 || sink) BPM_CUDA_TRY(cudaEventRecord(pl->ev_fork, s));

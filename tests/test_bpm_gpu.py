@@ -941,3 +941,39 @@ def test_plans_take_their_own_lock(bpm):
         stop.set()
         th.join()
     assert np.percentile(took, 80) < .25 * np.median(spent), (np.percentile(took, [50, 80, 95]), np.median(spent))
+
+
+def test_march_beside_another_callers_capture(bpm):
+    """While one caller captures a march in concurrent groups (the plan's streams are part of its
+    capture), another's march of the same plan on a stream of its own neither joins nor breaks the
+    capture: its groups follow one another there. Both give the bits of the march alone."""
+    import torch
+    kw = dict(units=(.1, .1, .1), lam=.5, n0=1.33, batch=4, use_graph=False, group=2, launch={"cluster": 2})
+    g = torch.Generator(device="cuda").manual_seed(3)
+    dn = .02 * torch.randn((6, 32, 64), device="cuda", generator=g)
+    a, b = (bpm.BatchedMarch((64, 32, 6), dn=dn, **kw) for _ in range(2))
+    assert a.plan is b.plan
+    u0 = torch.exp(1j * torch.rand((4, 32, 64), device="cuda", generator=g)).to(torch.complex64)
+    a.u0.copy_(u0)
+    b.u0.copy_(u0)
+    a.run()
+    torch.cuda.synchronize()
+    want = a.out.clone()
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    a.out.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        a.run()
+        b.run(side.cuda_stream)
+        a.run()
+    side.synchronize()
+    assert torch.equal(b.out, want)
+    assert not a.out.any()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(a.out, want)
+    b.out.zero_()
+    b.run(side.cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(b.out, want)
