@@ -278,7 +278,7 @@ def _check_shapes(size, u0, dn):
 def bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n_volumes=1, n0=1.,
            return_scattering=False, return_g=False, return_full=True, return_field=True,
            absorbing_width=0, use_fresnel_approx=False, scattering_plane_ind=0,
-           store_dn_as_half=False, mean_mode="weighted"):
+           store_dn_as_half=False, mean_mode="weighted", launch=None):
     """Simulates the propagation of a monochromatic wave of wavelength lam with initial
     field u0 along z through a medium of refractive index n0 + dn (bpm/bpm/bpm_3d.py:39).
 
@@ -287,6 +287,13 @@ def bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n_volumes=1, n0=1
     "simple" or "ignore". Returns the (Nz, Ny, Nx) complex field (return_field) or |u|^2
     volume, or only the last plane (return_full=False), plus (p[, g]) when
     return_scattering. n_volumes > 1 splits z into chunks as the reference does.
+
+    launch: a launch shape as bpm_3d_batched takes it. By default a march from 128 x 128 up may
+    be one launch that holds up to 128 SMs until it ends, so marches of several streams follow
+    one another; with {"cluster": 2} they interleave pass by pass. That pays for four or more
+    large marches at a time (GB300, ms for all, default against cluster = 2: four of 1024 x 1024
+    x 64 weighted 5.8 against 4.4, eight threads with one of 512 x 512 x 100 4.2 against 3.6),
+    not for one or two, nor at 256 x 256 and below (eight threads 2.1 against 2.7).
     """
     if n_volumes == 1:
         return _bpm_3d(size, units, lam=lam, u0=u0, dn=dn, subsample=subsample, n0=n0,
@@ -294,12 +301,12 @@ def bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n_volumes=1, n0=1
                        return_field=return_field, return_g=return_g, absorbing_width=absorbing_width,
                        use_fresnel_approx=use_fresnel_approx,
                        scattering_plane_ind=scattering_plane_ind,
-                       store_dn_as_half=store_dn_as_half, mean_mode=mean_mode)
+                       store_dn_as_half=store_dn_as_half, mean_mode=mean_mode, launch=launch)
     return _bpm_3d_split(size, units, lam=lam, u0=u0, dn=dn, n_volumes=n_volumes, subsample=subsample,
                          n0=n0, return_scattering=return_scattering, return_g=return_g,
                          absorbing_width=absorbing_width, return_full=return_full,
                          return_field=return_field, use_fresnel_approx=use_fresnel_approx,
-                         store_dn_as_half=store_dn_as_half, mean_mode=mean_mode)
+                         store_dn_as_half=store_dn_as_half, mean_mode=mean_mode, launch=launch)
 
 
 def _validate(mean_mode, subsample, return_scattering, return_g):
@@ -314,7 +321,7 @@ def _validate(mean_mode, subsample, return_scattering, return_g):
 def _bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n0=1.,
             return_scattering=False, return_g=False, return_full=True, return_field=True,
             use_fresnel_approx=False, absorbing_width=0, scattering_plane_ind=0,
-            return_last_plane=False, store_dn_as_half=False, mean_mode="weighted"):
+            return_last_plane=False, store_dn_as_half=False, mean_mode="weighted", launch=None):
     """One march over all of z (bpm/bpm/bpm_3d.py:_bpm_3d :104-423)."""
     _validate(mean_mode, subsample, return_scattering, return_g)
     Nx, Ny, Nz = (int(s) for s in size)
@@ -339,7 +346,7 @@ def _bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n0=1.,
     mask = precompute_mask(plan, dn_t, kind) if (dn_t is not None and mask_pays(1, Nx, Ny)) else None
     before = None if as_tensor else N.march_timeouts()
     out, last, p, g = _run(plan, u0_t, dn_t, kind, 0, out_kind, True, return_scattering, return_g,
-                           scattering_plane_ind, tabs, mask=mask)
+                           scattering_plane_ind, tabs, int((launch or {}).get("group", 0)), mask, launch)
     conv = (lambda t: t) if as_tensor else _d2h
     if return_full:
         res = conv(out[0])
@@ -360,7 +367,7 @@ def _bpm_3d(size, units, lam=.5, u0=None, dn=None, subsample=1, n0=1.,
 def _bpm_3d_split(size, units, lam=.5, u0=None, dn=None, n_volumes=1, n0=1., subsample=1,
                   return_scattering=False, return_full=True, return_g=False, return_field=True,
                   absorbing_width=0, use_fresnel_approx=False, store_dn_as_half=False,
-                  mean_mode="weighted"):
+                  mean_mode="weighted", launch=None):
     """z-chunked march (bpm/bpm/bpm_3d.py:_bpm_3d_split :863-992): chunks of Nz//n+1 planes
     with one plane of overlap, the last plane of a chunk handed on as the next u0. The
     per-chunk reference semantics are kept (in "weighted" mode each chunk reduces over its
@@ -383,7 +390,7 @@ def _bpm_3d_split(size, units, lam=.5, u0=None, dn=None, n_volumes=1, n0=1., sub
     kw = dict(units=units, lam=lam, n0=n0, subsample=subsample, return_full=return_full,
               return_field=return_field, return_g=return_g, absorbing_width=absorbing_width,
               return_scattering=return_scattering, store_dn_as_half=store_dn_as_half,
-              mean_mode=mean_mode, use_fresnel_approx=use_fresnel_approx)
+              mean_mode=mean_mode, use_fresnel_approx=use_fresnel_approx, launch=launch)
     for i in range(n_volumes):
         i1, i2 = i * Nz2, int(np.clip((i + 1) * Nz2, 0, Nz))
         if i < n_volumes - 1:

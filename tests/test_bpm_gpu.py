@@ -977,3 +977,22 @@ def test_march_beside_another_callers_capture(bpm):
     b.run(side.cuda_stream)
     torch.cuda.synchronize()
     assert torch.equal(b.out, want)
+
+
+@pytest.mark.parametrize("size,mode", [((256, 128, 9), "weighted"), ((256, 256, 6), "ignore"), ((128, 128, 7), "simple")])
+def test_single_march_takes_a_launch_shape(bpm, size, mode):
+    """bpm_3d's launch shape: with cluster = 2 a march beside others keeps to the pass kernels, the
+    same bits; scattering sums to FP32 rounding (they are added in another order)."""
+    Nx, Ny, Nz = size
+    rng = np.random.default_rng(Nx)
+    dn = (.03 * rng.standard_normal((Nz, Ny, Nx))).astype(np.float32)
+    kw = dict(lam=.5, n0=1.33, dn=dn, mean_mode=mode)
+    one = bpm.bpm_3d(size, (.1, .1, .1), **kw)
+    n0 = bpm.launch_count()
+    passes = bpm.bpm_3d(size, (.1, .1, .1), launch={"cluster": 2}, **kw)
+    assert bpm.launch_count() - n0 >= 2 * (Nz - 1)
+    assert np.array_equal(one, passes)
+    assert np.array_equal(one, bpm.bpm_3d(size, (.1, .1, .1), launch={}, **kw))
+    a = bpm.bpm_3d(size, (.1, .1, .1), return_scattering=True, launch={"cluster": 2}, **kw)
+    b = bpm.bpm_3d(size, (.1, .1, .1), return_scattering=True, **kw)
+    assert np.array_equal(a[0], b[0]) and rel_l2(a[1], b[1]) < 1e-6
