@@ -19,23 +19,23 @@ from .bpm3d import _apply_launch, _ptr, _stream_ptr, get_plan, mask_pays, precom
 
 __all__ = ["propagate_exit"]
 
-# A forward march whose planes take no more than this keeps them all instead of one in
-# ckpt_every, and its backward pass recomputes nothing: a third of the marching. GB300, 16
-# fields of 256x256x128 (1.07 GB): 5.32 -> 3.62 ms forward and backward.
+# A forward march that a backward pass will follow and whose planes take no more than this keeps
+# them all instead of one in ckpt_every, and the backward pass recomputes nothing: a third of the
+# marching. GB300, 16 fields of 256x256x128 (1.07 GB): 5.32 -> 3.62 ms forward and backward.
 KEEP_ALL_BYTES = 2 << 30
 
 
 class _ExitMarch(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx, dn, u0, plan, ckpt_every, group, launch):
+    def forward(ctx, dn, u0, plan, ckpt_every, group, launch, backward_follows):
         B, Ny, Nx = u0.shape
         Nz = plan.size[2]
         dev = u0.device
         u0c = u0.detach().to(torch.complex64).contiguous()
         dnc = dn.detach().to(torch.float32).contiguous() if dn is not None else None
         ckpt = None
-        if B * Nz * Ny * Nx * 8 <= KEEP_ALL_BYTES:
+        if backward_follows and B * Nz * Ny * Nx * 8 <= KEEP_ALL_BYTES:
             try:
                 ckpt = torch.empty((B, Nz, Ny, Nx), dtype=torch.complex64, device=dev)
                 ckpt_every = 1
@@ -101,7 +101,7 @@ class _ExitMarch(torch.autograd.Function):
         if ctx.has_dn and ctx.needs_input_grad[0]:
             gdn = grad_dn if (shared or ctx.bstride) else grad_dn.sum(dim=0)
             gdn = gdn.to(ctx.dn_dtype)
-        return gdn, grad_u0, None, None, None, None
+        return gdn, grad_u0, None, None, None, None, None
 
 
 def propagate_exit(dn, u0, size, units, lam=.5, n0=1., absorbing_width=0, ckpt_every=16,
@@ -123,4 +123,5 @@ def propagate_exit(dn, u0, size, units, lam=.5, n0=1., absorbing_width=0, ckpt_e
         raise ValueError("dn must have shape (..., %d, %d, %d)" % (Nz, Ny, Nx))
     if dn is not None and dn.is_complex():
         raise NotImplementedError("the adjoint needs real dn")
-    return _ExitMarch.apply(dn, u0, plan, int(ckpt_every), int(group), dict(launch or {}))
+    backward_follows = torch.is_grad_enabled() and (u0.requires_grad or (dn is not None and dn.requires_grad))
+    return _ExitMarch.apply(dn, u0, plan, int(ckpt_every), int(group), dict(launch or {}), backward_follows)

@@ -205,3 +205,39 @@ def test_kept_planes_equal_recomputed_ones(monkeypatch, fields, nx, ny, nz, ckpt
         got.append((out.detach(), dn.grad, u.grad))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def _case(fields, nx, ny, nz, grad):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(nz)
+    dn = (torch.rand((nz, ny, nx), device="cuda", generator=g) * .04).requires_grad_(grad)
+    u0 = torch.exp(1j * torch.rand((fields, ny, nx), device="cuda", generator=g)).to(torch.complex64)
+    return dn, u0
+
+
+def _peak(f):
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    r = f()
+    torch.cuda.synchronize()
+    return r, torch.cuda.max_memory_allocated() - before
+
+
+def test_forward_alone_does_not_keep_the_planes():
+    """Without a gradient to come (no_grad, or inputs that need none) the forward march writes one
+    plane in ckpt_every, not all of them; the exit planes are the same bits."""
+    import torch
+    from bpm_gb300 import adjoint
+    size, fields = (256, 256, 64), 4
+    planes = fields * 256 * 256 * 64 * 8
+    dn, u0 = _case(fields, *size, grad=True)
+    kept, held = _peak(lambda: adjoint.propagate_exit(dn, u0, size, (.1, .1, .1), .5, 1.33))
+    assert held > planes
+    with torch.no_grad():
+        a, peak_a = _peak(lambda: adjoint.propagate_exit(dn, u0, size, (.1, .1, .1), .5, 1.33))
+    b, peak_b = _peak(lambda: adjoint.propagate_exit(dn.detach(), u0, size, (.1, .1, .1), .5, 1.33))
+    assert peak_a < .7 * planes and peak_b < .7 * planes, (planes, held, peak_a, peak_b)
+    assert torch.equal(a, kept.detach()) and torch.equal(b, a) and not b.requires_grad
