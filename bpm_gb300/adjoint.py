@@ -25,6 +25,17 @@ __all__ = ["propagate_exit"]
 KEEP_ALL_BYTES = 2 << 30
 
 
+def _may_keep(planes, limit, dev):
+    """Whether a march may keep its planes (bytes) beyond the checkpoints asked for: within `limit`,
+    and within a sixteenth of the device memory that is free (by the driver, or in torch's cache),
+    so that several graphs alive at once, the march's own buffers and the caller's keep finding
+    room where one plane in ckpt_every left it. Up to 32 MB it does not ask (8 us)."""
+    if planes > limit or planes <= min(limit, 32 << 20):
+        return planes <= limit
+    free = torch.cuda.mem_get_info(dev)[0]
+    return 16 * planes <= free or 16 * planes <= free + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+
+
 class _ExitMarch(torch.autograd.Function):
 
     @staticmethod
@@ -35,7 +46,7 @@ class _ExitMarch(torch.autograd.Function):
         u0c = u0.detach().to(torch.complex64).contiguous()
         dnc = dn.detach().to(torch.float32).contiguous() if dn is not None else None
         ckpt = None
-        if backward_follows and B * Nz * Ny * Nx * 8 <= KEEP_ALL_BYTES:
+        if backward_follows and _may_keep(B * Nz * Ny * Nx * 8, launch.get("keep_bytes", KEEP_ALL_BYTES), dev):
             try:
                 ckpt = torch.empty((B, Nz, Ny, Nx), dtype=torch.complex64, device=dev)
                 ckpt_every = 1
@@ -111,7 +122,13 @@ def propagate_exit(dn, u0, size, units, lam=.5, n0=1., absorbing_width=0, ckpt_e
     in dn and u0 (torch autograd). prop = "functional" (bpm_3d, mean_mode="ignore") or
     "class" (Bpm3d's FP64 propagator). group and launch (keys conc, col_block; see
     bpm_gb300.autotune) set the launch shape of the forward and adjoint marches; they
-    change no result."""
+    change no result.
+
+    The march stores its field every ckpt_every planes and the backward pass recomputes the
+    planes between. Where a gradient is needed and all planes (8 bytes a voxel and field) take no
+    more than 2 GiB and a sixteenth of the free device memory, they are kept until the
+    backward pass instead, and nothing is recomputed; the launch key keep_bytes is another bound
+    than 2 GiB for this call, 0 for one plane in ckpt_every whatever is free."""
     kind = {"functional": N.PROP_FUNCTIONAL, "class": N.PROP_CLASS}[prop]
     plan = get_plan(size, units, lam, n0, absorbing_width, "ignore", kind)
     if u0.dim() == 2:

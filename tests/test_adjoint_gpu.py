@@ -241,3 +241,39 @@ def test_forward_alone_does_not_keep_the_planes():
     b, peak_b = _peak(lambda: adjoint.propagate_exit(dn.detach(), u0, size, (.1, .1, .1), .5, 1.33))
     assert peak_a < .7 * planes and peak_b < .7 * planes, (planes, held, peak_a, peak_b)
     assert torch.equal(a, kept.detach()) and torch.equal(b, a) and not b.requires_grad
+
+
+@pytest.mark.parametrize("how", ["little memory", "keep_bytes"])
+def test_kept_planes_are_bounded(monkeypatch, how):
+    """The planes are kept only where they take a sixteenth of the free device memory at most, and
+    no more than the call's own bound (launch key keep_bytes; 0: one plane in ckpt_every): the
+    gradients are the same bits, and what the graph holds is the checkpoints."""
+    import torch
+    from bpm_gb300 import adjoint
+    size, fields = (256, 256, 64), 4
+    planes = fields * 256 * 256 * 64 * 8
+    dn, u0 = _case(fields, *size, grad=True)
+
+    def grads(**kw):
+        out = adjoint.propagate_exit(dn, u0, size, (.1, .1, .1), .5, 1.33, **kw)
+        held = torch.cuda.memory_allocated()
+        return torch.autograd.grad((out.abs() ** 4).sum(), dn)[0], held
+
+    base = torch.cuda.memory_allocated()
+    want, held = grads()
+    assert held - base > planes
+    kw = {}
+    if how == "keep_bytes":
+        kw["launch"] = {"keep_bytes": 0}
+    else:
+        total = torch.cuda.mem_get_info()[1]
+        torch.cuda.empty_cache()
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (15 * planes, total))
+    base = torch.cuda.memory_allocated()
+    got, held = grads(**kw)
+    assert held - base < .7 * planes, (held - base, planes)
+    assert torch.equal(got, want)
+    if how == "keep_bytes":
+        again, held = grads(launch={"keep_bytes": planes})
+        assert torch.equal(again, want)
+        assert torch.equal(grads(launch={"keep_bytes": planes - 1})[0], want)
