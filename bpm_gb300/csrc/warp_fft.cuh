@@ -159,7 +159,7 @@ __device__ __forceinline__ void warp_fft_from(float2 (&v)[N / L], float2* buf, c
 // twiddle table (WarpFft<N, L>::TW entries, see wtw_offset).
 template <int N, bool INV, int L = 32>
 __device__ __forceinline__ void warp_fft(float2 (&v)[N / L], float2* buf, const float2* __restrict__ tw, int t) {
-  static_assert(N >= 64 && N <= 1024 && (L == 32 || L == 16 || L == 8), "warp FFT covers 64..1024 points");
+  static_assert(N >= 64 && N <= 1024 && (L == 32 || L == 16), "warp FFT covers 64..1024 points");
   warp_fft_from<N, 1, INV, L>(v, buf, tw, t);
 }
 

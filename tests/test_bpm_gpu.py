@@ -996,3 +996,35 @@ def test_single_march_takes_a_launch_shape(bpm, size, mode):
     a = bpm.bpm_3d(size, (.1, .1, .1), return_scattering=True, launch={"cluster": 2}, **kw)
     b = bpm.bpm_3d(size, (.1, .1, .1), return_scattering=True, **kw)
     assert np.array_equal(a[0], b[0]) and rel_l2(a[1], b[1]) < 1e-6
+
+
+@pytest.mark.parametrize("kind", ["f32", "c64"])
+def test_phase_sine_and_cosine_over_all_phases(bpm, kind):
+    """The masks of phases on both sides of 30000, where the march's own sine and cosine hand over to
+    sincosf, of zeros, subnormal and huge values, infinities and NaN, against FP64 values of the
+    float32 phase: 1.3e-7 (sincosf is good to 2 ulp, 1.2e-7 below 1; the other has 6.1e-8)."""
+    import torch
+    from bpm_gb300 import _native as N
+    from bpm_gb300.bpm3d import get_plan, precompute_mask
+    plan = get_plan((64, 64, 4), (.1, .1, .1), .5, 1.33, 0, "ignore")
+    uk = np.float32(2 * np.pi / .5 * .1)
+    rng = np.random.default_rng(5)
+    edge = np.float32(30000.) / uk
+    v = np.concatenate([rng.uniform(-3, 3, 5000), rng.uniform(-2e4, 2e4, 5000),
+                        edge * (1 + rng.uniform(-1e-5, 1e-5, 5000)) * rng.choice([-1, 1], 5000),
+                        10. ** rng.uniform(5, 37, 1374) * rng.choice([-1, 1], 1374),
+                        [0., -0., 1e-40, -1e-44, 3e38, -3e38, np.inf, -np.inf, np.nan, 1e-7]])
+    dn = np.resize(v.astype(np.float32), (4, 64, 64))
+    t = torch.from_numpy(dn).cuda()
+    if kind == "c64":
+        t = torch.complex(t, torch.zeros_like(t))
+    got = precompute_mask(plan, t, N.DN_C64 if kind == "c64" else N.DN_F32).cpu().numpy()
+    with np.errstate(over="ignore", invalid="ignore"):
+        x = ((-uk) * dn).astype(np.float32).astype(np.float64)
+        want = np.cos(x) + 1j * np.sin(x)
+    ok = np.isfinite(x)
+    assert (np.abs(x[ok]) > 30000).sum() > 1000 and (~ok).sum() >= 4
+    for a, b in ((got.real, want.real), (got.imag, want.imag)):
+        assert np.all(np.isnan(a[~ok]))
+        assert np.abs(a[ok] - b[ok]).max() < 1.3e-7
+    assert np.all(got[dn == 0.] == 1.)
