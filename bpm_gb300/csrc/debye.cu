@@ -712,8 +712,25 @@ __global__ void debye_point_nodes_kernel(NodeArgs a, double kz, float4* nd, floa
   }
 }
 
-// k r rounded to FP32: r^2 and r as float pairs (the error of each square by an FMA, one
-// Newton correction of the root), in FP64 where the squares would leave the FP32 range
+// x^2 + y^2 as a float pair: the error of each square by an FMA, that of their sum by a two-sum
+__device__ __forceinline__ float2 square_sum(float x, float y) {
+  const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), s = __fadd_rn(xx, yy);
+  const float bb = __fsub_rn(s, xx);
+  return make_float2(s, (__fsub_rn(xx, __fsub_rn(s, bb)) + __fsub_rn(yy, bb)) + (fmaf(x, x, -xx) + fmaf(y, y, -yy)));
+}
+// the root of a float pair as a float pair (one Newton correction)
+__device__ __forceinline__ float2 root_pair(float2 a) {
+  const float h = __fsqrt_rn(a.x);
+  return make_float2(h, __fdividef(fmaf(-h, h, a.x) + a.y, 2.f * h));
+}
+// the quotient of two float pairs, rounded once to FP32 (the remainder of the leading quotient is
+// exact in the FMA)
+__device__ __forceinline__ float div_pair(float2 n, float2 d) {
+  const float q = __fdiv_rn(n.x, d.x);
+  return __fadd_rn(q, __fdividef(fmaf(-q, d.x, n.x) + fmaf(-q, d.y, n.y), d.x));
+}
+
+// k r rounded to FP32, r a float pair, in FP64 where the squares would leave the FP32 range
 __device__ __forceinline__ float point_kr(float x, float y, const PointArgs& a) {
   if (x == 0.f && y == 0.f) return 0.f;
   const float m = fmaxf(fabsf(x), fabsf(y));
@@ -721,11 +738,25 @@ __device__ __forceinline__ float point_kr(float x, float y, const PointArgs& a) 
     const double xd = x, yd = y;
     return (float)(a.k * sqrt(xd * xd + yd * yd));
   }
-  const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), s = __fadd_rn(xx, yy);
-  const float bb = __fsub_rn(s, xx);
-  const float lo = (__fsub_rn(xx, __fsub_rn(s, bb)) + __fsub_rn(yy, bb)) + (fmaf(x, x, -xx) + fmaf(y, y, -yy));
-  const float h = __fsqrt_rn(s);
-  return mul_pair(make_float2(h, __fdividef(fmaf(-h, h, s) + lo, 2.f * h)), a.k2);
+  return mul_pair(root_pair(square_sum(x, y)), a.k2);
+}
+
+// (cos phi, sin phi, cos 2 phi, sin 2 phi) of a point's azimuth (phi = 0 at the origin) as x/r, y/r,
+// (x^2 - y^2)/r^2 and 2xy/r^2 of float pairs, each rounded once to FP32 as the FP64 values are
+// (quotients of plain floats were up to 2.5 roundings off). A power of two keeps the squares and
+// their errors in the FP32 range.
+__device__ __forceinline__ float4 point_azimuth(float x, float y) {
+  const float m = fmaxf(fabsf(x), fabsf(y));
+  if (!(m > 0.f)) return make_float4(1.f, 0.f, 1.f, 0.f);
+  const float sc = m < 0x1p-40f ? 0x1p100f : (m > 0x1p60f ? 0x1p-70f : 1.f);
+  x *= sc;
+  y *= sc;
+  const float2 r2 = square_sum(x, y), r = root_pair(r2);
+  const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), d = __fsub_rn(xx, yy), bb = __fsub_rn(d, xx);
+  const float dlo = (__fsub_rn(xx, __fsub_rn(d, bb)) - __fadd_rn(yy, bb)) + (fmaf(x, x, -xx) - fmaf(y, y, -yy));
+  const float xy = __fmul_rn(2.f * x, y);
+  return make_float4(div_pair(make_float2(x, 0.f), r), div_pair(make_float2(y, 0.f), r),
+                     div_pair(make_float2(d, dlo), r2), div_pair(make_float2(xy, fmaf(2.f * x, y, -xy)), r2));
 }
 
 // e^{i kz c} of a float pair c: the product as a pair (p, e), p reduced modulo 2 pi with the
@@ -815,17 +846,8 @@ __global__ void __launch_bounds__(PT_THREADS) debye_points_kernel(
     I2.y += __shfl_xor_sync(0xffffffffu, I2.y, o);
   }
   if (!active || sub != 0) return;
-  // azimuth from the coordinates scaled by their larger one (phi = 0 at the origin):
-  // cos phi = x/r, sin phi = y/r, cos 2 phi = (x-y)(x+y)/r^2, sin 2 phi = 2xy/r^2
-  float c1 = 1.f, s1 = 0.f, c2 = 1.f, s2 = 0.f;
-  const float m = fmaxf(fabsf(x), fabsf(y));
-  if (m > 0.f) {
-    const float xm = x / m, ym = y / m, r2 = fmaf(xm, xm, ym * ym), ir = rsqrtf(r2);
-    c1 = xm * ir;
-    s1 = ym * ir;
-    c2 = (xm - ym) * (xm + ym) / r2;
-    s2 = 2.f * xm * ym / r2;
-  }
+  const float4 az = point_azimuth(x, y);
+  const float c1 = az.x, s1 = az.y, c2 = az.z, s2 = az.w;
   const float ex0 = a.ex0, ey0 = a.ey0;
   // psf_debye.cl:254-263
   const float2 vx = make_float2(ex0 * (I0.x + I2.x * c2) + (ey0 * s2) * I2.x,

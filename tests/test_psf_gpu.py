@@ -328,3 +328,31 @@ def test_quadrature_accumulators(bpm, nz, steps):
     ref = debye_ref.focus_field_debye(*args, real_dtype=np.float64, complex_dtype=np.complex128)
     for a, b, k in zip(out, ref, ("u", "ex", "ey", "ez")):
         assert rel_l2(a, b) < TOL, k
+
+
+def test_azimuth_is_rounded_once(bpm):
+    """cos phi and sin 2 phi of free points to FP32 rounding of the FP64 values: points (x, y) of
+    whole-number right triangles with one hypotenuse share k r and so the integrals bit for bit.
+    Ez / Ez(r, 0) is cos phi within two roundings (2^-24 relative each: cos phi's own and the
+    product's); Ey / sin 2 phi is one number within two roundings a point."""
+    import torch
+    eps = 2.**-24
+    for r in (5 * 13 * 17 * 29 * 37, 5 * 13 * 17 * 29 * 41, 5 * 13 * 17 * 37 * 41, 5 * 13 * 29 * 37 * 41):
+        a = np.arange(1, r, dtype=np.int64)
+        b = np.rint(np.sqrt((r * r - a * a).astype(np.float64))).astype(np.int64)
+        ok = a * a + b * b == r * r
+        a, b = a[ok], b[ok]
+        assert len(a) > 200 and r < 2**23
+        for sc in (2.**-17, 2.**-110, 2.**-21):
+            x, y = (torch.from_numpy((np.concatenate([v, [w]]) * sc).astype(np.float32)).cuda()
+                    for v, w in ((a, r), (b, 0)))
+            # (the middle scale: radii far below the wavelength, in units that leave k r the same)
+            lam = .5 if sc != 2.**-110 else .5 * 2.**-93
+            _, _, ey, ez = bpm.focus_field_debye_at(x, y, torch.zeros_like(x), lam, .8, 1.33, 40, device=True)
+            ey, ez = ey.cpu().numpy().astype(np.complex128), ez.cpu().numpy().astype(np.complex128)
+            part = np.real if abs(ez[-1].real) > abs(ez[-1].imag) else np.imag
+            e = part(ez[:-1]) / part(ez[-1]) / (a / r) - 1
+            assert np.abs(e).max() < 2.01 * eps, (r, sc, np.abs(e).max() / eps)
+            part = np.real if abs(ey[0].real) > abs(ey[0].imag) else np.imag
+            q = part(ey[:-1]) / (2. * a * b / (float(r) * r))
+            assert q.max() - q.min() < 4.01 * eps * np.abs(q).max(), (r, sc, (q.max() - q.min()) / np.abs(q).max() / eps)
