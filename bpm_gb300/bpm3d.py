@@ -203,13 +203,14 @@ def _slice_tables(dn, n0, dev):
 def mask_pays(batch, Nx, Ny):
     """Whether a march of `batch` fields through one shared dn volume computes its phase
     masks once up front (precompute_mask) instead of per element in every row pass. The
-    results are the same bits either way. It pays for several fields, and for one field on
-    every grid measured, where the row pass stages one mask row instead of evaluating
-    exp/sincos per element (GB300, one field, precompute included, per-element -> mask:
-    Nz 128 ignore with complex dn 1024^2 4.74 -> 3.55 ms, 512^2 1.70 -> 1.23, 256^2 0.84 ->
-    0.74, 128^2 0.89 -> 0.81; weighted 1024^2 6.04 -> 5.01, 512^2 (Nz 256) 5.78 -> 4.57,
-    256^2 1.51 -> 1.38, 128^2 1.20 -> 1.13, 64^2 (Nz 64) 0.419 -> 0.405). Below 64x64 it
-    stays per element (not measured)."""
+    results are the same bits either way. It pays for several fields, and for one field up to
+    512^2 and on the pass kernels, whose row pass stages one mask row instead of evaluating
+    exp/sincos per element (GB300, one field, ms, precompute included, per element -> mask:
+    weighted 64^2 x 64 0.263 -> 0.235, 128^3 0.619 -> 0.572, 256^2 x 128 1.015 -> 0.982, 512^2 x
+    256 3.05 -> 2.93, ignore with complex dn 512^2 x 128 1.19 -> 1.13; on the pass kernels (launch
+    {"cluster": 2}) 512^2 5.30 -> 4.54, 1024^2 x 128 5.39 -> 4.45). One field of 1024^2 in one launch
+    forms its masks behind the gathering: 3.07 -> 3.15. Below 64x64 it stays per element (not
+    measured)."""
     return batch >= 2 or Nx * Ny >= 64 * 64
 
 
